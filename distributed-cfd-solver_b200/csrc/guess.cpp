@@ -44,8 +44,8 @@ Mlp::Mlp(int device, int nvars, uint64_t seed) : device_(device), nvars_(nvars) 
     v_ = dev_alloc<float>(kMlpParams, "mlp adam v");
     grad_ = dev_alloc<float>(kMlpParams, "mlp grad");
     loss_ = dev_alloc<float>(1, "mlp loss");
-    partials_ = dev_alloc<float>(static_cast<std::size_t>(grid_train_) * (kMlpParams + 1), "mlp partials");
-    w_ = dev_alloc<uint16_t>(kMlpHid * kMlpIn + kMlpHid * kMlpHid + kMlpOut * kMlpHid, "mlp bf16 weights");
+    partials_ = dev_alloc<float>(static_cast<std::size_t>(grid_train_) * kMlpPartials, "mlp partials");
+    w_ = dev_alloc<uint16_t>(kMlpWeights, "mlp bf16 weights");
     err_ = dev_alloc<int>(1, "mlp error flag");
     cuda_check(cudaMemset(m_, 0, kMlpParams * sizeof(float)), "memset");
     cuda_check(cudaMemset(v_, 0, kMlpParams * sizeof(float)), "memset");
@@ -65,15 +65,17 @@ Mlp::Mlp(int device, int nvars, uint64_t seed) : device_(device), nvars_(nvars) 
 Mlp::~Mlp() {
     for (void* q : {static_cast<void*>(params_), static_cast<void*>(m_), static_cast<void*>(v_),
                     static_cast<void*>(grad_), static_cast<void*>(loss_), static_cast<void*>(partials_),
-                    static_cast<void*>(w_), static_cast<void*>(err_)})
+                    static_cast<void*>(w_), static_cast<void*>(err_), static_cast<void*>(losses_)})
         if (q) cudaFree(q);
 }
 
 MlpDev Mlp::dev() const {
     MlpDev d;
     d.w1 = w_;
-    d.w2 = w_ + kMlpHid * kMlpIn;
-    d.w3 = w_ + kMlpHid * kMlpIn + kMlpHid * kMlpHid;
+    d.w2 = w_ + kMlpW2;
+    d.w3 = w_ + kMlpW3;
+    d.w2t = w_ + kMlpW2t;
+    d.w3t = w_ + kMlpW3t;
     d.params = params_;
     d.nout = nvars_;
     return d;
@@ -87,11 +89,14 @@ void Mlp::set_params(const float* p) {
         q[kOffB3 + o] = 0.0f;
     }
     cuda_check(cudaMemcpy(params_, q.data(), kMlpParams * sizeof(float), cudaMemcpyHostToDevice), "H2D");
-    std::vector<uint16_t> w(kMlpHid * kMlpIn + kMlpHid * kMlpHid + kMlpOut * kMlpHid);
-    std::size_t k = 0;
-    for (int i = 0; i < kMlpHid * kMlpIn; ++i) w[k++] = to_bf16(q[kOffW1 + i]);
-    for (int i = 0; i < kMlpHid * kMlpHid; ++i) w[k++] = to_bf16(q[kOffW2 + i]);
-    for (int i = 0; i < kMlpOut * kMlpHid; ++i) w[k++] = to_bf16(q[kOffW3 + i]);
+    std::vector<uint16_t> w(kMlpWeights);
+    for (int i = 0; i < kMlpHid * kMlpIn; ++i) w[i] = to_bf16(q[kOffW1 + i]);
+    for (int o = 0; o < kMlpHid; ++o)
+        for (int i = 0; i < kMlpHid; ++i)
+            w[kMlpW2 + o * kMlpHid + i] = w[kMlpW2t + i * kMlpHid + o] = to_bf16(q[kOffW2 + o * kMlpHid + i]);
+    for (int o = 0; o < kMlpOut; ++o)
+        for (int i = 0; i < kMlpHid; ++i)
+            w[kMlpW3 + o * kMlpHid + i] = w[kMlpW3t + i * kMlpOut + o] = to_bf16(q[kOffW3 + o * kMlpHid + i]);
     cuda_check(cudaMemcpy(w_, w.data(), w.size() * sizeof(uint16_t), cudaMemcpyHostToDevice), "H2D");
     step_ = 0;
     cuda_check(cudaMemset(m_, 0, kMlpParams * sizeof(float)), "memset");
@@ -118,18 +123,19 @@ void Mlp::forward(const uint16_t* feat, int64_t rows, const double* scale, doubl
     cuda_check(cudaGetLastError(), "mlp forward launch");
 }
 
-float Mlp::run_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, float lr, cudaStream_t s) {
+void Mlp::queue_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, float lr, float* loss_dev,
+                     cudaStream_t s) {
     if (rows <= 0) throw Failure{CFDG_ERR_INVALID, "empty batch"};
-    launch_mlp_grad(dev(), X, T, rows, partials_, err_, grid_train_, s);
+    const int parts = launch_mlp_grad(dev(), X, T, rows, partials_, err_, grid_train_, s);
     if (adam) ++step_;
     const double inv = 1.0 / (double(rows) * nvars_);
-    uint16_t* w1 = w_;
-    uint16_t* w2 = w_ + kMlpHid * kMlpIn;
-    uint16_t* w3 = w2 + kMlpHid * kMlpHid;
-    launch_mlp_adam(params_, m_, v_, w1, w2, w3, partials_, grid_train_, inv, lr, 0.9f, 0.999f, 1e-8f,
-                    std::max(step_, 1), adam, grad_, loss_, s);
-    launches_ += adam ? 3 : 2;
+    launch_mlp_adam(params_, m_, v_, w_, partials_, parts, inv, lr, 0.9f, 0.999f, 1e-8f, std::max(step_, 1), adam,
+                    grad_, loss_dev, s);
+    launches_ += 2;
     cuda_check(cudaGetLastError(), "mlp train launch");
+}
+
+float Mlp::read_loss(cudaStream_t s) {
     float loss = 0.0f;
     cuda_check(cudaMemcpyAsync(&loss, loss_, sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     check_err(s);
@@ -137,7 +143,8 @@ float Mlp::run_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, 
 }
 
 float Mlp::gradient(const uint16_t* X, const float* T, int64_t rows, float* grad_host, cudaStream_t s) {
-    const float loss = run_grad(X, T, rows, false, 0.0f, s);
+    queue_grad(X, T, rows, false, 0.0f, loss_, s);
+    const float loss = read_loss(s);
     if (grad_host) {
         cuda_check(cudaMemcpyAsync(grad_host, grad_, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
         cuda_check(cudaStreamSynchronize(s), "sync");
@@ -146,7 +153,8 @@ float Mlp::gradient(const uint16_t* X, const float* T, int64_t rows, float* grad
 }
 
 float Mlp::adam_step(const uint16_t* X, const float* T, int64_t rows, float lr, cudaStream_t s) {
-    return run_grad(X, T, rows, true, lr, s);
+    queue_grad(X, T, rows, true, lr, loss_, s);
+    return read_loss(s);
 }
 
 float Mlp::train(const Dataset& ds, int epochs, int batch, float lr, uint64_t seed, cudaStream_t s) {
@@ -158,14 +166,30 @@ float Mlp::train(const Dataset& ds, int epochs, int batch, float lr, uint64_t se
     std::vector<int64_t> order(static_cast<std::size_t>(nb));
     std::iota(order.begin(), order.end(), int64_t(0));
     std::mt19937_64 g(seed);
+    // the batches of an epoch follow one another on the stream; the host
+    // reads their losses and the error flag once per epoch
+    if (losses_cap_ < nb) {
+        if (losses_) cudaFree(losses_);
+        losses_ = nullptr;
+        losses_cap_ = 0;
+        losses_ = dev_alloc<float>(static_cast<std::size_t>(nb), "mlp batch losses");
+        losses_cap_ = nb;
+    }
+    std::vector<float> host(static_cast<std::size_t>(nb));
     float last = 0.0f;
     for (int e = 0; e < epochs; ++e) {
         std::shuffle(order.begin(), order.end(), g);
-        double acc = 0.0;
         for (int64_t k : order) {
             const int64_t r0 = k * batch, rows = std::min<int64_t>(batch, n - r0);
-            acc += double(adam_step(ds.X() + r0 * kMlpIn, ds.T() + r0 * kMlpOut, rows, lr, s)) * double(rows);
+            queue_grad(ds.X() + r0 * kMlpIn, ds.T() + r0 * kMlpOut, rows, true, lr, losses_ + k, s);
         }
+        cuda_check(cudaMemcpyAsync(host.data(), losses_, sizeof(float) * static_cast<std::size_t>(nb),
+                                   cudaMemcpyDeviceToHost, s),
+                   "D2H");
+        check_err(s);
+        double acc = 0.0;
+        for (int64_t k : order)
+            acc += double(host[static_cast<std::size_t>(k)]) * double(std::min<int64_t>(batch, n - k * batch));
         last = static_cast<float>(acc / double(n));
     }
     return last;

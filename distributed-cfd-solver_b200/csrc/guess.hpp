@@ -52,12 +52,17 @@ private:
     float* grad_ = nullptr;
     float* loss_ = nullptr;
     float* partials_ = nullptr;
-    uint16_t* w_ = nullptr;  // bf16 W1 | W2 | W3
+    uint16_t* w_ = nullptr;  // bf16 copies (kMlpWeights)
     int* err_ = nullptr;
+    float* losses_ = nullptr;  // losses of an epoch's batches
+    int64_t losses_cap_ = 0;
     int grid_train_ = 1, grid_fwd_ = 1;
     int step_ = 0;
     int64_t launches_ = 0;
-    float run_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, float lr, cudaStream_t s);
+    // gradient and optional Adam step of a batch; its loss goes to *loss_dev
+    void queue_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, float lr, float* loss_dev,
+                    cudaStream_t s);
+    float read_loss(cudaStream_t s);
     void check_err(cudaStream_t s);
 };
 

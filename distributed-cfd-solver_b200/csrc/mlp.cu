@@ -39,14 +39,6 @@ __device__ void load_tile(uint8_t* tile, const uint16_t* __restrict__ g, int R, 
     }
 }
 
-// Transposed load: tile element (r, k) = g[k * R + r] (g row-major [K x R]).
-__device__ void load_tile_t(uint8_t* tile, const uint16_t* __restrict__ g, int R, int K) {
-    for (int q = threadIdx.x; q < R * K; q += blockDim.x) {
-        const int r = q / K, k = q - r * K;
-        *reinterpret_cast<uint16_t*>(tile + tc::core_offset(r, k, K)) = g[int64_t(k) * R + r];
-    }
-}
-
 __device__ void zero_bytes(uint8_t* p, int bytes) {
     for (int q = threadIdx.x; q < bytes / 16; q += blockDim.x)
         reinterpret_cast<uint4*>(p)[q] = make_uint4(0u, 0u, 0u, 0u);
@@ -211,6 +203,31 @@ __device__ __forceinline__ uint64_t epi_hidden(uint32_t tacc, const float* bias,
     return mask;
 }
 
+// As epi_hidden, and the transposed activations into rows 0..63 of `ht`
+// (column = this thread's sample), straight from the registers.
+__device__ __forceinline__ void put_bf16(uint8_t* tile, int r, int k, int K, float v) {
+    *reinterpret_cast<uint16_t*>(tile + tc::core_offset(r, k, K)) = f2bf(v);
+}
+__device__ __forceinline__ uint64_t epi_hidden_t(uint32_t tacc, const float* bias, uint8_t* h, uint8_t* ht) {
+    const int r = threadIdx.x;
+    uint64_t mask = 0;
+#pragma unroll
+    for (int c = 0; c < 64; c += 16) {
+        float v[16];
+        tc::tmem_ld16(lane_base(tacc) + c, v);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float z = v[i] + bias[c + i];
+            if (z > 0.0f) mask |= (uint64_t(1) << (c + i));
+            v[i] = fmaxf(z, 0.0f);
+            put_bf16(ht, c + i, r, 128, v[i]);
+        }
+        store8(h, r, c, 64, v);
+        store8(h, r, c + 8, 64, v + 8);
+    }
+    return mask;
+}
+
 // ----------------------------------------------------------- inference
 __global__ void __launch_bounds__(128) k_mlp_forward(MlpDev net, const uint16_t* __restrict__ feat, int64_t rows,
                                                      const double* __restrict__ scale, int nv,
@@ -314,21 +331,26 @@ __device__ TrainSmem carve_train(uint8_t* smem) {
     return s;
 }
 
-__device__ __forceinline__ void put_bf16(uint8_t* tile, int r, int k, int K, float v) {
-    *reinterpret_cast<uint16_t*>(tile + tc::core_offset(r, k, K)) = f2bf(v);
-}
-
+// Gradient of one batch.  A batch is a few tiles a CTA (8,192 samples: 64 tiles
+// of 128), so the time is the set-up, the chain of seven products with their
+// epilogues, and the partials' store, not the tensor cores: the weights come
+// in as 16-byte words in both orientations, the transposed operands are
+// written from registers, and the partials leave as 16-byte words.  With the
+// losses read once an epoch, one epoch of 8,192-sample batches over 600,011
+// samples went from 5.0 to 1.75 ms (68 to 24 us a batch).
 __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t* __restrict__ feat,
                                                      const float* __restrict__ target, int64_t rows,
                                                      float* __restrict__ partials, int* err) {
     extern __shared__ __align__(128) uint8_t smem[];
     const TrainSmem s = carve_train(smem);
+    if (__syncthreads_or(*err != 0)) return;  // an earlier batch failed: the host reports it
     load_net(net, s.w1, s.w2, s.w3, s.bias);
-    load_tile_t(s.w2t, net.w2, kMlpHid, kMlpHid);  // (in, out) = W2[out][in]
-    load_tile_t(s.w3t, net.w3, kMlpHid, kMlpOut);  // (in, out) = W3[out][in]
-    zero_bytes(s.xt, 16384);
-    zero_bytes(s.h1t, 20480);
-    zero_bytes(s.at, 32768);
+    load_tile(s.w2t, net.w2t, kMlpHid, kMlpHid, kMlpHid);  // (in, out)
+    load_tile(s.w3t, net.w3t, kMlpHid, kMlpOut, kMlpHid);
+    // the padding rows of the transposed operands (8 rows of 128: 2 KB)
+    zero_bytes(s.xt + 6 * 2048, 2 * 2048);
+    zero_bytes(s.h1t + 8 * 2048, 2 * 2048);
+    zero_bytes(s.at + 8 * 2048, 8 * 2048);
     __syncthreads();
     for (int k = threadIdx.x; k < 128; k += blockDim.x) {
         put_bf16(s.xt, 48, k, 128, 1.0f);
@@ -354,13 +376,30 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int64_t r0 = t * kMlpTile;
         const bool valid = r0 + r < rows;
-        // X and X^T (row r = sample; padded samples are zero and carry no loss)
-        load_tile(s.x, feat + r0 * kMlpIn, kMlpTile, kMlpIn, rows - r0);
-        __syncthreads();
-        for (int q = threadIdx.x; q < kMlpTile * kMlpIn; q += blockDim.x) {
-            const int smp = q / kMlpIn, f = q - smp * kMlpIn;
-            const uint16_t v = *reinterpret_cast<const uint16_t*>(s.x + tc::core_offset(smp, f, kMlpIn));
-            *reinterpret_cast<uint16_t*>(s.xt + tc::core_offset(f, smp, 128)) = v;
+        // X and X^T (row r = sample; padded samples are zero and carry no loss),
+        // and the sample's targets, which the output layer needs
+        uint4 xv[kMlpIn / 8];
+        float tv[kMlpOut];
+#pragma unroll
+        for (int c = 0; c < kMlpIn / 8; ++c)
+            xv[c] = valid ? __ldg(reinterpret_cast<const uint4*>(feat + (r0 + r) * kMlpIn) + c) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int c = 0; c < kMlpOut / 4; ++c) {
+            const float4 q = valid ? __ldg(reinterpret_cast<const float4*>(target + (r0 + r) * kMlpOut) + c)
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+            tv[4 * c] = q.x;
+            tv[4 * c + 1] = q.y;
+            tv[4 * c + 2] = q.z;
+            tv[4 * c + 3] = q.w;
+        }
+#pragma unroll
+        for (int c = 0; c < kMlpIn / 8; ++c) {
+            *reinterpret_cast<uint4*>(s.x + tc::core_offset(r, c * 8, kMlpIn)) = xv[c];
+            const uint32_t u[4] = {xv[c].x, xv[c].y, xv[c].z, xv[c].w};
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                *reinterpret_cast<uint16_t*>(s.xt + tc::core_offset(c * 8 + i, r, 128)) =
+                    static_cast<uint16_t>(u[i >> 1] >> ((i & 1) * 16));
         }
         to_mma();
         if (r == 0) {
@@ -368,27 +407,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
             tc::mma_commit(s.bar);
         }
         if (!wait_all(s.bar, phase, err)) return abort_tc(s.bar, phase, tb, 512);
-        const uint64_t m1 = epi_hidden(tb + kT1, s.bias, s.h);
-        // H1^T for dW2
-        for (int q = threadIdx.x; q < kMlpTile * kMlpHid; q += blockDim.x) {
-            const int smp = q / kMlpHid, j = q - smp * kMlpHid;
-            const uint16_t v = *reinterpret_cast<const uint16_t*>(s.h + tc::core_offset(smp, j, kMlpHid));
-            *reinterpret_cast<uint16_t*>(s.h1t + tc::core_offset(j, smp, 128)) = v;
-        }
+        const uint64_t m1 = epi_hidden_t(tb + kT1, s.bias, s.h, s.h1t);  // H1 and H1^T (of dW2)
         to_mma();
         if (r == 0) {
             issue_gemm(tb + kT2, s.h, s.w2, 64, kMlpHid, false);
             tc::mma_commit(s.bar);
         }
         if (!wait_all(s.bar, phase, err)) return abort_tc(s.bar, phase, tb, 512);
-        const uint64_t m2 = epi_hidden(tb + kT2, s.bias + 64, s.h);
-        __syncthreads();
-        // H2^T for dW3^T (rows 0..63 of the shared transposed tile)
-        for (int q = threadIdx.x; q < kMlpTile * kMlpHid; q += blockDim.x) {
-            const int smp = q / kMlpHid, j = q - smp * kMlpHid;
-            const uint16_t v = *reinterpret_cast<const uint16_t*>(s.h + tc::core_offset(smp, j, kMlpHid));
-            *reinterpret_cast<uint16_t*>(s.at + tc::core_offset(j, smp, 128)) = v;
-        }
+        const uint64_t m2 = epi_hidden_t(tb + kT2, s.bias + 64, s.h, s.at);  // H2 and H2^T (of dW3^T)
         to_mma();
         if (r == 0) {
             issue_gemm(tb + kT1, s.h, s.w3, 16, kMlpHid, false);
@@ -402,7 +428,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
 #pragma unroll
             for (int v = 0; v < 16; ++v) {
                 float d = 0.0f;
-                if (valid && v < nout) d = (y[v] + s.bias[128 + v]) - target[(r0 + r) * kMlpOut + v];
+                if (valid && v < nout) d = (y[v] + s.bias[128 + v]) - tv[v];
                 dy[v] = d;
                 loss += d * d;
             }
@@ -455,11 +481,14 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
         // the H2^T rows of s.at are rewritten by the next tile: restore nothing
         // (row 64 keeps its ones, rows 65.. stay zero)
     }
-    // write this CTA's gradient partials (zero when it processed no tile)
-    float* P = partials + int64_t(blockIdx.x) * (kMlpParams + 1);
-    if (first) {
-        for (int p = threadIdx.x; p < kMlpParams; p += blockDim.x) P[p] = 0.0f;
-    } else {
+    // write this CTA's gradient partials (the grid has no CTA without a tile)
+    float* P = partials + int64_t(blockIdx.x) * kMlpPartials;
+    auto put16 = [](float* dst, const float* v) {
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+            *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    };
+    {
         float v[16];
         // dW3^T: row r = input unit (r < 64), row 64 = db3
         tc::tmem_ld16(lane_base(tb + kGW3), v);
@@ -472,23 +501,19 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
 #pragma unroll
         for (int c = 0; c < 64; c += 16) {
             tc::tmem_ld16(lane_base(tb + kGW1) + c, v);
-            if (r < 64)
-                for (int i = 0; i < 16; ++i) {
-                    const int col = c + i;
-                    if (col < kMlpIn) P[kOffW1 + r * kMlpIn + col] = v[i];
-                    else if (col == kMlpIn) P[kOffB1 + r] = v[i];
-                }
+            if (r < 64) {
+                if (c < kMlpIn) put16(P + kOffW1 + r * kMlpIn + c, v);
+                else P[kOffB1 + r] = v[0];
+            }
         }
         // dW2: row r = output unit, columns 0..63 inputs, 64 bias
 #pragma unroll
         for (int c = 0; c < 80; c += 16) {
             tc::tmem_ld16(lane_base(tb + kGW2) + c, v);
-            if (r < 64)
-                for (int i = 0; i < 16; ++i) {
-                    const int col = c + i;
-                    if (col < kMlpHid) P[kOffW2 + r * kMlpHid + col] = v[i];
-                    else if (col == kMlpHid) P[kOffB2 + r] = v[i];
-                }
+            if (r < 64) {
+                if (c < kMlpHid) put16(P + kOffW2 + r * kMlpHid + c, v);
+                else P[kOffB2 + r] = v[0];
+            }
         }
     }
     // loss partial (fixed-order block sum)
@@ -507,13 +532,30 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
     }
 }
 
-__global__ void k_mlp_adam(float* params, float* m, float* v, const float* __restrict__ partials, int nparts,
-                           double inv_count, float lr, float b1, float b2, float eps, float c1, float c2, bool adam,
-                           float* grad_out, float* loss_out) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > kMlpParams) return;
-    double acc = 0.0;
-    for (int c = 0; c < nparts; ++c) acc += double(partials[int64_t(c) * (kMlpParams + 1) + p]);
+// One Adam step.  kAdamSlices threads share a parameter: slice q adds the
+// CTAs q, q + kAdamSlices, ... in order, the slices' sums follow one another.
+// The updated weights leave in bf16 as well, in both orientations the products
+// read.  Bound by the latency of the partials' loads (a few MB in L2).
+constexpr int kAdamParams = 32, kAdamSlices = 8;
+
+__global__ void __launch_bounds__(kAdamParams * kAdamSlices)
+    k_mlp_adam(float* params, float* m, float* v, uint16_t* __restrict__ w, const float* __restrict__ partials,
+               int nparts, double inv_count, float lr, float b1, float b2, float eps, float c1, float c2, bool adam,
+               float* grad_out, float* loss_out) {
+    __shared__ double sh[kAdamSlices][kAdamParams];
+    const int local = threadIdx.x % kAdamParams, slice = threadIdx.x / kAdamParams;
+    const int p = blockIdx.x * kAdamParams + local;
+    double part = 0.0;
+    if (p <= kMlpParams) {
+#pragma unroll 8
+        for (int c = slice; c < nparts; c += kAdamSlices) part += double(__ldg(partials + int64_t(c) * kMlpPartials + p));
+    }
+    sh[slice][local] = part;
+    __syncthreads();
+    if (slice != 0 || p > kMlpParams) return;
+    double acc = sh[0][local];
+#pragma unroll
+    for (int q = 1; q < kAdamSlices; ++q) acc += sh[q][local];
     if (p == kMlpParams) {
         if (loss_out) *loss_out = float(acc * inv_count);
         return;
@@ -525,14 +567,20 @@ __global__ void k_mlp_adam(float* params, float* m, float* v, const float* __res
     const float vi = b2 * v[p] + (1.0f - b2) * g * g;
     m[p] = mi;
     v[p] = vi;
-    params[p] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-__global__ void k_mlp_sync_bf16(const float* __restrict__ params, uint16_t* w1, uint16_t* w2, uint16_t* w3) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kMlpHid * kMlpIn) w1[i] = f2bf(params[kOffW1 + i]);
-    if (i < kMlpHid * kMlpHid) w2[i] = f2bf(params[kOffW2 + i]);
-    if (i < kMlpOut * kMlpHid) w3[i] = f2bf(params[kOffW3 + i]);
+    const float x = params[p] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    params[p] = x;
+    const uint16_t h = f2bf(x);
+    if (p < kOffB1) {
+        w[p - kOffW1] = h;
+    } else if (p >= kOffW2 && p < kOffB2) {
+        const int q = p - kOffW2, o = q / kMlpHid, i = q - o * kMlpHid;
+        w[kMlpW2 + q] = h;
+        w[kMlpW2t + i * kMlpHid + o] = h;
+    } else if (p >= kOffW3 && p < kOffB3) {
+        const int q = p - kOffW3, o = q / kMlpHid, i = q - o * kMlpHid;
+        w[kMlpW3 + q] = h;
+        w[kMlpW3t + i * kMlpOut + o] = h;
+    }
 }
 
 }  // namespace
@@ -552,23 +600,21 @@ void launch_mlp_forward(const MlpDev& net, const uint16_t* feat, int64_t rows, c
     k_mlp_forward<<<g, 128, kFwdSmem, s>>>(net, feat, rows, scale, nv, out, err);
 }
 
-void launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target, int64_t rows, float* partials,
-                     int* err, int grid, cudaStream_t s) {
+int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target, int64_t rows, float* partials,
+                    int* err, int grid, cudaStream_t s) {
     cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
-    k_mlp_grad<<<grid, 128, kTrainSmem, s>>>(net, feat, target, rows, partials, err);
+    const int64_t ntiles = (rows + kMlpTile - 1) / kMlpTile;
+    const int g = static_cast<int>(std::min<int64_t>(ntiles, grid));
+    k_mlp_grad<<<g, 128, kTrainSmem, s>>>(net, feat, target, rows, partials, err);
+    return g;
 }
 
-void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w1, uint16_t* w2, uint16_t* w3,
-                     const float* partials, int nparts, double inv_count, float lr, float beta1, float beta2,
-                     float eps, int step, bool adam, float* grad_out, float* loss_out, cudaStream_t s) {
+void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials, int nparts,
+                     double inv_count, float lr, float beta1, float beta2, float eps, int step, bool adam,
+                     float* grad_out, float* loss_out, cudaStream_t s) {
     const float c1 = 1.0f - powf(beta1, float(step)), c2 = 1.0f - powf(beta2, float(step));
-    k_mlp_adam<<<(kMlpParams + 1 + 255) / 256, 256, 0, s>>>(params, m, v, partials, nparts, inv_count, lr, beta1,
-                                                             beta2, eps, c1, c2, adam, grad_out, loss_out);
-    if (adam) launch_mlp_sync_bf16(params, w1, w2, w3, s);
-}
-
-void launch_mlp_sync_bf16(const float* params, uint16_t* w1, uint16_t* w2, uint16_t* w3, cudaStream_t s) {
-    k_mlp_sync_bf16<<<(kMlpHid * kMlpHid + 255) / 256, 256, 0, s>>>(params, w1, w2, w3);
+    k_mlp_adam<<<(kMlpParams + kAdamParams) / kAdamParams, kAdamParams * kAdamSlices, 0, s>>>(
+        params, m, v, w, partials, nparts, inv_count, lr, beta1, beta2, eps, c1, c2, adam, grad_out, loss_out);
 }
 
 }  // namespace cfdg

@@ -23,12 +23,20 @@ constexpr int kOffB2 = kOffW2 + kMlpHid * kMlpHid;
 constexpr int kOffW3 = kOffB2 + kMlpHid;
 constexpr int kOffB3 = kOffW3 + kMlpOut * kMlpHid;
 constexpr int kMlpParams = kOffB3 + kMlpOut;  // 8336
+// floats of one CTA's gradient partials: the parameters, the loss, padded to
+// whole 16-byte words
+constexpr int kMlpPartials = (kMlpParams + 1 + 3) / 4 * 4;
+// bf16 copies: W1 | W2 | W3 | W2^T | W3^T
+constexpr int kMlpW2 = kMlpHid * kMlpIn, kMlpW3 = kMlpW2 + kMlpHid * kMlpHid, kMlpW2t = kMlpW3 + kMlpOut * kMlpHid,
+              kMlpW3t = kMlpW2t + kMlpHid * kMlpHid, kMlpWeights = kMlpW3t + kMlpHid * kMlpOut;
 
 // Device views of the network used by the kernels.
 struct MlpDev {
     const uint16_t* w1;  // bf16 bits, row-major out x in
     const uint16_t* w2;
     const uint16_t* w3;
+    const uint16_t* w2t;  // row-major in x out
+    const uint16_t* w3t;
     const float* params;  // fp32 master (biases are read from here)
     int nout;             // outputs that carry a loss (nvars)
 };
@@ -43,17 +51,16 @@ void launch_mlp_forward(const MlpDev& net, const uint16_t* feat, int64_t rows, c
                         double* out, int* err, int grid, cudaStream_t s);
 
 // Loss and gradient partials of mean squared error over `rows` samples:
-// partials[cta * (kMlpParams + 1) + p], last entry the CTA's loss sum.
-void launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target, int64_t rows, float* partials,
-                     int* err, int grid, cudaStream_t s);
+// partials[cta * kMlpPartials + p], entry kMlpParams the CTA's loss sum.  Runs
+// on at most `grid` CTAs and returns how many wrote partials.
+int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target, int64_t rows, float* partials,
+                    int* err, int grid, cudaStream_t s);
 
 // Sums the CTA partials in fixed order, scales by 1/(rows * nout), and
-// applies one Adam step (or only writes the gradient when adam == false).
-void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w1, uint16_t* w2, uint16_t* w3,
-                     const float* partials, int nparts, double inv_count, float lr, float beta1, float beta2,
-                     float eps, int step, bool adam, float* grad_out, float* loss_out, cudaStream_t s);
-
-// Rounds the fp32 master weights to the bf16 copies.
-void launch_mlp_sync_bf16(const float* params, uint16_t* w1, uint16_t* w2, uint16_t* w3, cudaStream_t s);
+// applies one Adam step, refreshing the bf16 copies `w` (or only writes the
+// gradient when adam == false).
+void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials, int nparts,
+                     double inv_count, float lr, float beta1, float beta2, float eps, int step, bool adam,
+                     float* grad_out, float* loss_out, cudaStream_t s);
 
 }  // namespace cfdg

@@ -76,6 +76,25 @@ def test_gradient_matches_oracle(cb, nvars, rows):
         assert np.linalg.norm(g[s:e] - g_ref[s:e]) <= 3e-2 * max(np.linalg.norm(g_ref[s:e]), 1e-30)
 
 
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128 + 1])
+def test_gradient_at_tile_edges(cb, rows):
+    """One sample, a tile with and without padding, a second tile, and one
+    more tile than a grid of one CTA per SM takes at once.  Tolerances as for
+    the gradient above; a single sample's gradient is a few units' bf16
+    rounding, 5e-2."""
+    nvars = 6
+    p = _params(5, nvars)
+    X = _features(cb, 6, rows)
+    T = np.zeros((rows, M.OUT), dtype=np.float32)
+    T[:, :nvars] = np.random.default_rng(7).standard_normal((rows, nvars))
+    net = cb.Mlp(nvars, seed=1)
+    net.set_params(p)
+    loss, g = net.gradient(X, T)
+    loss_ref, g_ref = M.loss_and_grad(p, M.from_bits(X), T.astype(np.float64), nvars)
+    assert abs(loss - loss_ref) <= 1e-4 * abs(loss_ref)
+    assert np.linalg.norm(g - g_ref) <= (5e-2 if rows == 1 else 2e-2) * np.linalg.norm(g_ref)
+
+
 def test_training_fits_a_teacher(cb):
     nvars, rows = 5, 24576
     teacher = _params(11, nvars)
