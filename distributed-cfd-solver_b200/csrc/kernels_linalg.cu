@@ -479,6 +479,173 @@ __global__ void __launch_bounds__(256) k_sgs_level_coop(BsrView A, const MT* __r
     }
 }
 
+// The level-scheduled sweep of a system whose z fits in the shared memory of
+// one thread-block cluster.  A level takes the latency of its barrier and of
+// one row's dependent loads, and the grid-wide barrier and the round trips
+// through L2 made that 4.4 us (204 levels of the 16k-cell plate).  Here z lives in the cluster's
+// distributed shared memory (row i in CTA i mod C), the barrier is the
+// cluster's, and everything of a warp's next row that does not depend on z
+// (blocks, columns, r, LU factors, pivots) is loaded before the barrier.  One
+// cluster has the bandwidth for it: the levels of such a system hold a few
+// hundred rows.  The arithmetic of a row is k_sgs_level_coop's to the bit: one
+// lane group per off-diagonal block, the products subtracted in ascending
+// column order, the pivoted substitution.  3.2 us a level on the same plate
+// (a sweep 0.96 -> 0.66 ms).
+constexpr int kClusterThreads = 512;
+constexpr int kClusterWarps = kClusterThreads / 32;
+
+template <typename MT, int BS>
+struct LevelRow {  // a row's data that does not depend on z; two blocks per lane group ahead
+    int4 rec;      // row, first block, end, diagonal block
+    double a0[BS], a1[BS], r, lu0, lu1;
+    int32_t c0, c1;
+    int piv;
+};
+
+template <typename MT, int BS>
+__global__ void __launch_bounds__(kClusterThreads)
+    k_sgs_level_cluster(BsrView A, const MT* __restrict__ vals, const MT* __restrict__ lu,
+                        const int8_t* __restrict__ piv, const int4* __restrict__ fwd_rows,
+                        const int32_t* __restrict__ fwd_off, int n_fwd, const int4* __restrict__ bwd_rows,
+                        const int32_t* __restrict__ bwd_off, int n_bwd, const double* __restrict__ r, double* z,
+                        int from_zero, const int* __restrict__ active) {
+    if (active && *active != 0) return;  // the same value for every CTA
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int KS = 32 / BS, B2 = BS * BS;
+    extern __shared__ __align__(16) double zs[];
+    __shared__ double lu_s[kClusterWarps][B2];
+    __shared__ int8_t piv_s[kClusterWarps][8];
+    const int C = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
+    const int shift = __ffs(C) - 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp = lane / BS, ii = lane - grp * BS;
+    const bool in_grp = grp < KS;
+    const int gl = in_grp ? grp * BS : 0;  // first lane of the group
+    const int gwarp = warp * C + rank, nwarps = kClusterWarps * C;
+    for (int e = threadIdx.x; e < (A.n - rank + C - 1) / C * BS; e += kClusterThreads) {
+        const int q = e / BS;
+        zs[e] = from_zero ? 0.0 : z[(int64_t(q) * C + rank) * BS + (e - q * BS)];
+    }
+    // the k-th off-diagonal block of the row in rec
+    auto off_block = [](const int4& rec, int q) { return rec.y + q + (rec.y + q >= rec.w ? 1 : 0); };
+    auto fetch = [&](const int4* rows, int32_t slot) {
+        LevelRow<MT, BS> w;
+        w.rec = __ldg(rows + slot);
+        const int m = w.rec.z - w.rec.y - 1;
+        w.c0 = w.c1 = 0;
+        if (in_grp && grp < m) {
+            const int32_t k = off_block(w.rec, grp);
+            w.c0 = __ldg(A.cols + k);
+            load_block_row<MT, BS>(vals + int64_t(k) * B2 + ii * BS, w.a0);
+        }
+        if (in_grp && KS + grp < m) {
+            const int32_t k = off_block(w.rec, KS + grp);
+            w.c1 = __ldg(A.cols + k);
+            load_block_row<MT, BS>(vals + int64_t(k) * B2 + ii * BS, w.a1);
+        }
+        const int64_t i = w.rec.x;
+        w.r = grp == 0 ? __ldg(r + i * BS + ii) : 0.0;
+        w.lu0 = lane < B2 ? ld(lu + i * B2 + lane) : 0.0;
+        w.lu1 = lane + 32 < B2 ? ld(lu + i * B2 + lane + 32) : 0.0;
+        w.piv = lane < BS ? piv[i * BS + lane] : 0;
+        return w;
+    };
+    // t = A_k[ii][:] . z_col of this lane's block; each lane of the group
+    // reads one entry of z_col and the group exchanges them
+    auto block_product = [&](const double (&a)[BS], int32_t c, bool on) {
+        double x = 0.0;
+        if (on) x = cluster.map_shared_rank(zs, c & (C - 1))[(c >> shift) * BS + ii];
+        double t = 0.0;
+#pragma unroll
+        for (int jj = 0; jj < BS; ++jj) {
+            const double xj = __shfl_sync(0xffffffffu, x, gl + jj);
+            if (on) t += a[jj] * xj;
+        }
+        return t;
+    };
+    auto solve = [&](const LevelRow<MT, BS>& w, bool last) {
+        const int m = w.rec.z - w.rec.y - 1;
+        if (lane < B2) lu_s[warp][lane] = w.lu0;
+        if (lane + 32 < B2) lu_s[warp][lane + 32] = w.lu1;
+        if (lane < BS) piv_s[warp][lane] = static_cast<int8_t>(w.piv);
+        double s = w.r;
+        for (int q0 = 0; q0 < m; q0 += KS) {
+            const int q = q0 + grp;
+            const bool on = in_grp && q < m;
+            double t;
+            if (q0 == 0) {
+                t = block_product(w.a0, w.c0, on);
+            } else if (q0 == KS) {
+                t = block_product(w.a1, w.c1, on);
+            } else {  // long rows: the blocks beyond the ones fetched ahead
+                double a[BS] = {};
+                int32_t c = 0;
+                if (on) {
+                    const int32_t k = off_block(w.rec, q);
+                    c = __ldg(A.cols + k);
+                    load_block_row<MT, BS>(vals + int64_t(k) * B2 + ii * BS, a);
+                }
+                t = block_product(a, c, on);
+            }
+#pragma unroll
+            for (int g = 0; g < KS; ++g) {
+                const double tg = __shfl_sync(0xffffffffu, t, g * BS + (ii < BS ? ii : 0));
+                if (q0 + g < m) s -= tg;
+            }
+        }
+        double b[BS];
+#pragma unroll
+        for (int j = 0; j < BS; ++j) b[j] = __shfl_sync(0xffffffffu, s, j);
+        __syncwarp();
+        if (grp == 0) {
+            lu_solve<double, BS, true>(lu_s[warp], piv_s[warp], b);
+            double out = b[0];
+#pragma unroll
+            for (int j = 1; j < BS; ++j)
+                if (j == ii) out = b[j];
+            const int32_t i = w.rec.x;
+            cluster.map_shared_rank(zs, i & (C - 1))[(i >> shift) * BS + ii] = out;
+            if (last) z[int64_t(i) * BS + ii] = out;
+        }
+        __syncwarp();
+    };
+    cluster.sync();  // z in place
+    // this warp's rows in order: (pass, level, slot); the next one is fetched
+    // before the barrier that ends the current level
+    int pass = 0, g = 0;
+    int32_t slot = fwd_off[0] + gwarp;
+    auto seek = [&] {  // moves to the next level that holds `slot`'s index for this warp
+        while (pass < 2) {
+            const int32_t* off = pass ? bwd_off : fwd_off;
+            const int ng = pass ? n_bwd : n_fwd;
+            while (g < ng && slot >= __ldg(off + g + 1)) {
+                ++g;
+                if (g < ng) slot = __ldg(off + g) + gwarp;
+            }
+            if (g < ng) return;
+            ++pass;
+            g = 0;
+            if (pass < 2) slot = __ldg(bwd_off) + gwarp;
+        }
+    };
+    seek();
+    LevelRow<MT, BS> w{};
+    if (pass < 2) w = fetch(pass ? bwd_rows : fwd_rows, slot);
+    for (int ps = 0; ps < 2; ++ps) {
+        const int ng = ps ? n_bwd : n_fwd;
+        for (int lv = 0; lv < ng; ++lv) {
+            while (pass == ps && g == lv) {
+                solve(w, ps == 1);
+                slot += nwarps;
+                seek();
+                if (pass < 2) w = fetch(pass ? bwd_rows : fwd_rows, slot);
+            }
+            cluster.sync();
+        }
+    }
+}
+
 // The last backward pass of a split multicolour sweep (colour 0, rows
 // [0, n_rows), every neighbour of a later colour and already final) fused
 // with the product y = A z on those rows.  The pass computes
@@ -903,6 +1070,81 @@ bool launch_sgs_level_coop(const BsrView& A, const MT* vals, const MT* lu, const
     if (grid <= 0) return false;
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, 0, s) == cudaSuccess;
 }
+
+// The cluster that holds z of n rows in shared memory (C CTAs, smem bytes
+// each), 0 when none does.  16 CTAs is the largest cluster (opt-in size).
+template <typename MT, int BS>
+static int level_cluster(int32_t n, int* smem) {
+    constexpr int kBytes = 200 * 1024;  // of 227 KB; the kernel's static arrays take up to 4.7 KB
+    for (int C : {16, 8}) {
+        const int64_t bytes = (int64_t(n) + C - 1) / C * BS * 8;
+        if (bytes > kBytes) continue;
+        auto* fn = k_sgs_level_cluster<MT, BS>;
+        if (C > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+        }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(C);
+        cfg.blockDim = dim3(kClusterThreads);
+        cfg.dynamicSmemBytes = static_cast<std::size_t>(bytes);
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = C;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int active = 0;
+        if (cudaOccupancyMaxActiveClusters(&active, fn, &cfg) != cudaSuccess || active < 1) {
+            cudaGetLastError();
+            continue;
+        }
+        *smem = static_cast<int>(bytes);
+        return C;
+    }
+    return 0;
+}
+
+int sgs_level_cluster(int32_t n, int bs, bool mixed, int* smem) {
+    if (n <= 0) return 0;
+    if (bs == 5) return mixed ? level_cluster<float, 5>(n, smem) : level_cluster<double, 5>(n, smem);
+    if (bs == 6) return mixed ? level_cluster<float, 6>(n, smem) : level_cluster<double, 6>(n, smem);
+    return 0;
+}
+
+template <typename MT>
+bool launch_sgs_level_cluster(const BsrView& A, const MT* vals, const MT* lu, const int8_t* piv, const int4* fwd_rows,
+                              const int32_t* fwd_off, int n_fwd, const int4* bwd_rows, const int32_t* bwd_off,
+                              int n_bwd, const double* r, double* z, bool from_zero, int C, int smem,
+                              const int* active, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(C);
+    cfg.blockDim = dim3(kClusterThreads);
+    cfg.dynamicSmemBytes = static_cast<std::size_t>(smem);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    const int zero = from_zero ? 1 : 0;
+    if (A.bs == 5)
+        return cudaLaunchKernelEx(&cfg, k_sgs_level_cluster<MT, 5>, A, vals, lu, piv, fwd_rows, fwd_off, n_fwd,
+                                  bwd_rows, bwd_off, n_bwd, r, z, zero, active) == cudaSuccess;
+    return cudaLaunchKernelEx(&cfg, k_sgs_level_cluster<MT, 6>, A, vals, lu, piv, fwd_rows, fwd_off, n_fwd, bwd_rows,
+                              bwd_off, n_bwd, r, z, zero, active) == cudaSuccess;
+}
+template bool launch_sgs_level_cluster<double>(const BsrView&, const double*, const double*, const int8_t*,
+                                               const int4*, const int32_t*, int, const int4*, const int32_t*, int,
+                                               const double*, double*, bool, int, int, const int*, cudaStream_t);
+template bool launch_sgs_level_cluster<float>(const BsrView&, const float*, const float*, const int8_t*, const int4*,
+                                              const int32_t*, int, const int4*, const int32_t*, int, const double*,
+                                              double*, bool, int, int, const int*, cudaStream_t);
 
 int dot_blocks(int64_t len) { return static_cast<int>(vec_grid(len)); }
 

@@ -64,6 +64,16 @@ template <typename MT>
 bool launch_sgs_level_coop(const BsrView& A, const MT* vals, const MT* lu, const int8_t* piv, const int4* fwd_rows,
                            const int32_t* fwd_off, int n_fwd, const int4* bwd_rows, const int32_t* bwd_off,
                            int n_bwd, const double* r, double* z, const int* active, cudaStream_t s);
+// The same sweep for a system whose z fits in the shared memory of one
+// cluster: sgs_level_cluster gives the cluster's CTAs and their shared-memory
+// bytes (0: it does not fit, or block sizes other than 5 and 6).  from_zero:
+// z starts from zero (else from the array); z is written once at the end.
+int sgs_level_cluster(int32_t n, int bs, bool mixed, int* smem);
+template <typename MT>
+bool launch_sgs_level_cluster(const BsrView& A, const MT* vals, const MT* lu, const int8_t* piv, const int4* fwd_rows,
+                              const int32_t* fwd_off, int n_fwd, const int4* bwd_rows, const int32_t* bwd_off,
+                              int n_bwd, const double* r, double* z, bool from_zero, int C, int smem,
+                              const int* active, cudaStream_t s);
 void launch_krylov_init(int64_t len, const double* b, const double* v, double* r, double* r0, double* p,
                         double* partials, KrylovScalars* ks, cudaStream_t s);
 // After launch_krylov_init: a rejected initial guess (||b - A x0|| >=

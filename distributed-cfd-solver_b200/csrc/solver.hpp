@@ -224,6 +224,7 @@ private:
     DevArray<int32_t> fwd_off_d_, bwd_off_d_;  // level boundaries on the device (cooperative level sweep)
     DevArray<int4> fwd_meta_, bwd_meta_;       // (row, first block, block end, diagonal) in level order
     bool level_coop_ = true;                  // cleared when the cooperative launch is unavailable
+    int level_cluster_ = 0, level_smem_ = 0;  // level sweep in one cluster: CTAs (0: not used), shared memory each
     double spmv_bytes(int n_extra_vectors, bool read_y) const;
     // rows [fwd_off_[1], n) of a colour-ordered matrix: block count and
     // distinct columns (the SpMV left after the fused colour-0 product)
