@@ -22,7 +22,45 @@ struct KrylovScalars {
     double rel_tol, abs_tol;
     double bnorm, scale, tol, initial, rnorm;
     double rho, rho_old, rho_new, alpha, omega, omega_new, beta;
+    // Solves reduced to the rows outside the first colour
+    // (kernels_reduced.cu): the caller's vectors, the arrival counter of the
+    // grid sums, the updates x has had, |rho_0|^2 and the colour-0
+    // multiples of rho_0 in r, p and s (cp_new: p after the update).
+    double* x;
+    const double* b;
+    unsigned arrived;
+    int updates;
+    double q0, cr, cp, cp_new, cs;
 };
+
+// A multicolour system for the reduced BiCGSTAB: colour 0 at positions
+// [0, n0), colour 1 at [n0, n1).  Position = row (rows null) when the rows are
+// in colour order, else rows[position] with two colours.  mid[row]: first
+// block outside the colour-0 columns (rows in colour order only).
+struct RedView {
+    int32_t n, n0, n1, bs;
+    const int32_t *row_ptr, *cols, *diag, *mid, *rows;
+};
+enum : int { RED_BACK0, RED_BACK, RED_FWD, RED_ETA, RED_WSUM, RED_XRED };
+int red_partials();  // doubles of the reduction buffer
+// r0 = b - A x (v = A x; null: x = 0), r and p on the rest rows, the scalars
+void launch_red_init(const RedView& A, KrylovScalars* ks, const double* v, double* r, double* r0, double* p,
+                     double* partials, bool guess, cudaStream_t st);
+// One sweep pass over the positions [pos0, pos1); second: the s vector's
+// sweep (cs), else the p vector's (cp)
+template <typename MT>
+void launch_red_sweep(const RedView& A, const MT* vals, const double* dinv, int kind, int32_t pos0, int32_t pos1,
+                      const double* src, const double* w, double* z, double* e, const KrylovScalars* ks, bool second,
+                      cudaStream_t st);
+template <typename MT>
+void launch_red_product(const RedView& A, const MT* vals, const double* src, const double* e, double* out,
+                        const double* r0, KrylovScalars* ks, double* partials, bool first, cudaStream_t st);
+void launch_red_s(const RedView& A, const double* dinv, const double* r, const double* v, const double* w, double* s,
+                  double* z, const KrylovScalars* ks, cudaStream_t st);
+void launch_red_update(const RedView& A, const double* dinv, const double* zs, const double* s, const double* t,
+                       const double* v, const double* w, double* r, double* p, double* zp, KrylovScalars* ks,
+                       double* partials, cudaGraphConditionalHandle cond, bool use_cond, cudaStream_t st);
+void launch_red_enter(const KrylovScalars* ks, cudaGraphConditionalHandle cond, cudaStream_t st);
 
 // Up to five (a, b) vector pairs; a null pointer stands for the SpMV output.
 struct DotSpec {

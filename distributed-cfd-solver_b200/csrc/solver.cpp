@@ -255,15 +255,19 @@ BsrSystem::BsrSystem(int device, int32_t n, int32_t bs, const int32_t* row_ptr, 
     // the fused colour-0 product and the SpMV of the other rows write their
     // partials one after the other
     alloc_or_throw(partials_,
-                   static_cast<std::size_t>(sgs_last_spmv_blocks(n, bs) + std::max(dot_blocks(N), spmv_blocks(n, bs))) * 5 + 8,
+                   std::max(static_cast<std::size_t>(sgs_last_spmv_blocks(n, bs) + std::max(dot_blocks(N), spmv_blocks(n, bs))) * 5,
+                            static_cast<std::size_t>(red_partials())) + 8,
                    "partials");
     alloc_or_throw(ks_, 1, "krylov scalars");
     alloc_or_throw(err_, 1, "error flag");
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_host_), sizeof(KrylovScalars)), "cudaMallocHost");
+    cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_init_), sizeof(KrylovScalars)), "cudaMallocHost");
 }
 
 BsrSystem::~BsrSystem() {
     release_device_loop();
+    release_red_graphs();
+    if (ks_init_) cudaFreeHost(ks_init_);
     if (ks_host_) cudaFreeHost(ks_host_);
     if (gm_h_host_) cudaFreeHost(gm_h_host_);
 }
@@ -272,7 +276,8 @@ void BsrSystem::set_precision(int precision) {
     if (precision != CFDG_PREC_FP64 && precision != CFDG_PREC_MIXED) throw Failure{CFDG_ERR_INVALID, "unknown precision"};
     if (precision == precision_) return;
     const std::size_t nv = static_cast<std::size_t>(nnzb_) * bs_ * bs_;
-    release_device_loop();  // the captured iteration launches precision-specific kernels
+    release_device_loop();  // the captured iterations launch precision-specific kernels
+    release_red_graphs();
     if (precision == CFDG_PREC_MIXED) {
         vals64_.release();
         lu64_.release();
@@ -280,6 +285,7 @@ void BsrSystem::set_precision(int precision) {
     } else {
         vals32_.release();
         lu32_.release();
+        dinv64_.release();
         alloc_or_throw(vals64_, nv, "values");
     }
     precision_ = precision;
@@ -356,19 +362,48 @@ void BsrSystem::build_ordering(int ordering) {
             bwd_key[i] = l;
         }
     } else {
-        std::vector<int32_t> color(n, -1);
+        std::vector<int32_t> color;
         std::vector<char> used;
         int32_t ncol = 0;
-        for (int32_t i = 0; i < n; ++i) {
-            used.assign(static_cast<std::size_t>(ncol) + 1, 0);
-            for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) {
-                const int32_t j = cols_h_[k];
-                if (j != i && color[j] >= 0) used[color[j]] = 1;
+        // smallest colour free among the row's columns and, once needed, the
+        // rows that list it (`lists`)
+        std::vector<int32_t> loff, lists;
+        auto colour_rows = [&] {
+            color.assign(n, -1);
+            ncol = 0;
+            for (int32_t i = 0; i < n; ++i) {
+                used.assign(static_cast<std::size_t>(ncol) + 1, 0);
+                for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) {
+                    const int32_t j = cols_h_[k];
+                    if (j != i && color[j] >= 0) used[color[j]] = 1;
+                }
+                if (!lists.empty())
+                    for (int32_t k = loff[i]; k < loff[i + 1]; ++k)
+                        if (lists[k] != i && color[lists[k]] >= 0) used[color[lists[k]]] = 1;
+                int32_t c = 0;
+                while (used[c]) ++c;
+                color[i] = c;
+                ncol = std::max(ncol, c + 1);
             }
-            int32_t c = 0;
-            while (used[c]) ++c;
-            color[i] = c;
-            ncol = std::max(ncol, c + 1);
+        };
+        auto coupled = [&] {
+            for (int32_t i = 0; i < n; ++i)
+                for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k)
+                    if (cols_h_[k] != i && color[cols_h_[k]] == color[i]) return true;
+            return false;
+        };
+        colour_rows();
+        // a pattern that is not symmetric can leave rows of a colour coupled:
+        // colour against the transposed pattern too
+        if (coupled()) {
+            loff.assign(static_cast<std::size_t>(n) + 1, 0);
+            for (int32_t j : cols_h_) ++loff[j + 1];
+            for (int32_t i = 0; i < n; ++i) loff[i + 1] += loff[i];
+            lists.resize(cols_h_.size());
+            std::vector<int32_t> cur(loff.begin(), loff.end() - 1);
+            for (int32_t i = 0; i < n; ++i)
+                for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) lists[cur[cols_h_[k]]++] = i;
+            colour_rows();
         }
         for (int32_t i = 0; i < n; ++i) {
             fwd_key[i] = color[i];
@@ -407,6 +442,61 @@ void BsrSystem::build_ordering(int ordering) {
     // sweep can split each row at its diagonal (k_sgs_rows MODE 2 / 3)
     split_ = ordering == CFDG_SGS_COLOR;
     for (std::size_t g = 0; split_ && g < fwd_first_.size(); ++g) split_ = fwd_first_[g] == fwd_off_[g];
+    // Reduced BiCGSTAB (kernels_reduced.cu): at least two colours, and rows in
+    // colour order, or two colours, where every off-diagonal block of a row
+    // is of the other colour.
+    const int ncolor = static_cast<int>(fwd_off_.size()) - 1;
+    reducible_ = reduce != REDUCE_NONE && ordering == CFDG_SGS_COLOR && ncolor >= 2 && (split_ || ncolor == 2);
+    if (reducible_) {
+        std::vector<int32_t> mid(n);
+        for (int32_t i = 0; i < n; ++i) {
+            int32_t k = row_ptr_h_[i];
+            while (k < diag_h_[i] && fwd_key[cols_h_[k]] == 0) ++k;
+            mid[i] = k;
+        }
+        upload_or_throw(mid_, mid, stream_, "sgs row splits");
+        cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // mid dies here
+        if (!w_.p) alloc_or_throw(w_, static_cast<std::size_t>(n) * bs_, "krylov");
+    }
+    release_red_graphs();
+    // the passes' byte counts are formed when a profiler asks for them
+    bytes_counted_ = false;
+    for (int m = 0; m < 3; ++m) {
+        fwd_bytes_[m].assign(fwd_off_.size() - 1, 0.0);
+        fwd_blocks_[m].assign(fwd_off_.size() - 1, 0.0);
+        bwd_bytes_[m].assign(bwd_off_.size() - 1, 0.0);
+        bwd_blocks_[m].assign(bwd_off_.size() - 1, 0.0);
+    }
+    red_back_.assign(fwd_off_.size() - 1, PassCount{});
+    red_fwd_.assign(fwd_off_.size() - 1, PassCount{});
+    upload_or_throw(fwd_rows_, fr, stream_, "sgs rows");
+    upload_or_throw(bwd_rows_, br, stream_, "sgs rows");
+    upload_or_throw(fwd_off_d_, fwd_off_, stream_, "sgs levels");
+    upload_or_throw(bwd_off_d_, bwd_off_, stream_, "sgs levels");
+    if (ordering == CFDG_SGS_LEVEL) {
+        auto meta = [&](const std::vector<int32_t>& rows) {
+            std::vector<int4> m(rows.size());
+            for (std::size_t q = 0; q < rows.size(); ++q) {
+                const int32_t i = rows[q];
+                m[q] = make_int4(i, row_ptr_h_[i], row_ptr_h_[i + 1], diag_h_[i]);
+            }
+            return m;
+        };
+        upload_or_throw(fwd_meta_, meta(fr), stream_, "sgs level rows");
+        upload_or_throw(bwd_meta_, meta(br), stream_, "sgs level rows");
+    }
+    level_cluster_ = ordering == CFDG_SGS_LEVEL ? sgs_level_cluster(n, bs_, precision_ == CFDG_PREC_MIXED, &level_smem_) : 0;
+    cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // the host vectors are rebuilt by the next call
+    fwd_rows_h_ = std::move(fr);
+    bwd_rows_h_ = std::move(br);
+    ordering_ = ordering;
+}
+
+// Blocks and unique-touch bytes of every pass of the ordering (profiling).
+void BsrSystem::count_pass_bytes() {
+    const int32_t n = n_;
+    const int ordering = ordering_;
+    const std::vector<int32_t>&fr = fwd_rows_h_, &br = bwd_rows_h_;
     rest_nnzb_ = rest_cols_ = 0.0;
     if (split_ && fwd_off_.size() > 2) {
         std::vector<char> used(n, 0);
@@ -414,6 +504,42 @@ void BsrSystem::build_ordering(int ordering) {
             for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) used[cols_h_[k]] = 1;
         for (int32_t j = 0; j < n; ++j) rest_cols_ += used[j];
         rest_nnzb_ = double(nnzb_ - row_ptr_h_[fwd_off_[1]]);
+    }
+    if (reducible_) {
+        const int ncolor = groups_fwd();
+        std::vector<int32_t> fwd_key(n), seen(n, -1);
+        for (int g = 0; g < ncolor; ++g)
+            for (int32_t q = fwd_off_[g]; q < fwd_off_[g + 1]; ++q) fwd_key[fr[q]] = g;
+        int32_t stamp = 0;
+        // blocks (and distinct vector entries) of the rows of colours
+        // [g0, g1) whose column's colour is in [c0, c1)
+        auto count = [&](int g0, int g1, auto&& range) {
+            PassCount c;
+            ++stamp;
+            for (int32_t q = fwd_off_[g0]; q < fwd_off_[g1]; ++q) {
+                const int32_t i = fr[q];
+                const auto [c0, c1] = range(fwd_key[i]);
+                c.rows += 1.0;
+                for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) {
+                    const int32_t kc = fwd_key[cols_h_[k]];
+                    if (cols_h_[k] == i || kc < c0 || kc >= c1) continue;
+                    c.blocks += 1.0;
+                    if (seen[cols_h_[k]] != stamp) {
+                        seen[cols_h_[k]] = stamp;
+                        c.entries += 1.0;
+                    }
+                }
+            }
+            return c;
+        };
+        red_back_.clear();
+        red_fwd_.clear();
+        for (int g = 0; g < ncolor; ++g) {
+            red_back_.push_back(count(g, g + 1, [&](int c) { return std::pair<int, int>(c + 1, ncolor); }));
+            red_fwd_.push_back(count(g, g + 1, [&](int c) { return std::pair<int, int>(1, c); }));
+        }
+        red_lower_ = count(1, ncolor, [&](int c) { return std::pair<int, int>(0, c); });
+        red_w_ = count(1, ncolor, [&](int) { return std::pair<int, int>(0, 1); });
     }
     // Unique-touch bytes of one pass over a group: row list, row pointers,
     // diagonal index, off-diagonal blocks + columns, LU + pivots, r (or the
@@ -463,43 +589,30 @@ void BsrSystem::build_ordering(int ordering) {
     };
     pass_bytes(fwd_off_, fr, true, fwd_bytes_, fwd_blocks_);
     pass_bytes(bwd_off_, br, false, bwd_bytes_, bwd_blocks_);
-    upload_or_throw(fwd_rows_, fr, stream_, "sgs rows");
-    upload_or_throw(bwd_rows_, br, stream_, "sgs rows");
-    upload_or_throw(fwd_off_d_, fwd_off_, stream_, "sgs levels");
-    upload_or_throw(bwd_off_d_, bwd_off_, stream_, "sgs levels");
-    if (ordering == CFDG_SGS_LEVEL) {
-        auto meta = [&](const std::vector<int32_t>& rows) {
-            std::vector<int4> m(rows.size());
-            for (std::size_t q = 0; q < rows.size(); ++q) {
-                const int32_t i = rows[q];
-                m[q] = make_int4(i, row_ptr_h_[i], row_ptr_h_[i + 1], diag_h_[i]);
-            }
-            return m;
-        };
-        upload_or_throw(fwd_meta_, meta(fr), stream_, "sgs level rows");
-        upload_or_throw(bwd_meta_, meta(br), stream_, "sgs level rows");
-    }
-    level_cluster_ = ordering == CFDG_SGS_LEVEL ? sgs_level_cluster(n, bs_, precision_ == CFDG_PREC_MIXED, &level_smem_) : 0;
-    cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // the host vectors are rebuilt by the next call
-    ordering_ = ordering;
+    bytes_counted_ = true;
 }
 
 void BsrSystem::sgs_setup(int ordering, int sweeps) {
     if (ordering != CFDG_SGS_LEVEL && ordering != CFDG_SGS_COLOR) throw Failure{CFDG_ERR_INVALID, "unknown SGS ordering"};
     if (sweeps < 1) throw Failure{CFDG_ERR_INVALID, "SGS sweeps must be >= 1"};
     if (ordering != ordering_) build_ordering(ordering);
+    if (prof_->on() && !bytes_counted_) count_pass_bytes();
     sweeps_ = sweeps;
     const std::size_t nb2 = static_cast<std::size_t>(n_) * bs_ * bs_;
     if (!piv_.p && n_ > 0) alloc_or_throw(piv_, static_cast<std::size_t>(n_) * bs_, "pivots");
     cuda_check(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_), "memset");
+    const bool color = ordering_ == CFDG_SGS_COLOR;
+    const double b2 = double(bs_) * bs_;
     if (precision_ == CFDG_PREC_MIXED) {
+        const bool inv64 = color && reducible();
         if (!lu32_.p && n_ > 0) alloc_or_throw(lu32_, nb2, "lu");
-        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (bs_ * bs_ * 8.0 + bs_ + 4.0));
-        launch_lu_setup<float>(view(), vals32_.p, lu32_.p, piv_.p, err_.p, ordering_ == CFDG_SGS_COLOR, stream_);
+        if (inv64 && !dinv64_.p) alloc_or_throw(dinv64_, nb2, "diagonal inverses");
+        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * (8.0 + (inv64 ? 8.0 : 0.0)) + bs_ + 4.0));
+        launch_lu_setup<float>(view(), vals32_.p, lu32_.p, inv64 ? dinv64_.p : nullptr, piv_.p, err_.p, color, stream_);
     } else {
         if (!lu64_.p && n_ > 0) alloc_or_throw(lu64_, nb2, "lu");
-        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (bs_ * bs_ * 16.0 + bs_ + 4.0));
-        launch_lu_setup<double>(view(), vals64_.p, lu64_.p, piv_.p, err_.p, ordering_ == CFDG_SGS_COLOR, stream_);
+        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + bs_ + 4.0));
+        launch_lu_setup<double>(view(), vals64_.p, lu64_.p, nullptr, piv_.p, err_.p, color, stream_);
     }
     cuda_check(cudaGetLastError(), "lu launch");
     int err = 0;
@@ -676,10 +789,232 @@ void BsrSystem::release_device_loop() {
     loop_exec_ = nullptr;
 }
 
+// ------------------------------------------------------- reduced BiCGSTAB
+RedView BsrSystem::red_view() const {
+    return RedView{n_,          fwd_off_[1], fwd_off_[2], bs_, row_ptr_.p, cols_.p,
+                   diag_.p,     mid_.p,      split_ ? nullptr : fwd_rows_.p};
+}
+
+// Blocks, columns, row structure, D^-1 rows and full-row vectors of a pass.
+double BsrSystem::red_bytes(const PassCount& c, double dinv_rows, double vectors) const {
+    return c.blocks * (block_bytes() + 4.0) + c.rows * 12.0 + c.entries * bs_ * 8.0 +
+           dinv_rows * bs_ * bs_ * 8.0 + vectors * c.rows * bs_ * 8.0;
+}
+
+// r = b - A x (the product already in v_ unless x = 0), w, and the first
+// step of the first sweep.
+template <typename MT>
+void BsrSystem::red_begin_t(const MT* vals, const double* dinv, Start start) {
+    const RedView R = red_view();
+    const double N = double(n_) * bs_, n0 = R.n0;
+    {
+        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, start == START_GUESS ? 2 : 1,
+                     8.0 * N * (start == START_ZERO ? 3.0 : 4.0));
+        launch_red_init(R, ks_.p, start == START_ZERO ? nullptr : v_.p, r_.p, r0_.p, p_.p, partials_.p,
+                        start == START_GUESS, stream_);
+    }
+    {
+        ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 3,
+                     n0 * bs_ * (bs_ * 8.0 + 16.0) + red_bytes(red_w_, 0.0, 1.0) +
+                         red_bytes(PassCount{red_fwd_[1].rows, 0.0, 0.0}, red_fwd_[1].rows, 3.0));
+        launch_red_sweep<MT>(R, vals, dinv, RED_ETA, 0, R.n0, r0_.p, nullptr, nullptr, t_.p, ks_.p, false, stream_);
+        launch_red_sweep<MT>(R, vals, dinv, RED_WSUM, R.n0, n_, nullptr, nullptr, w_.p, t_.p, ks_.p, false, stream_);
+        launch_red_sweep<MT>(R, vals, dinv, RED_FWD, R.n0, R.n1, p_.p, w_.p, phat_.p, nullptr, ks_.p, false, stream_);
+    }
+}
+
+// out = A M^-1 src on the rest rows with the inner products; z holds the
+// sweep of colour 1 on entry and M^-1 src (rest rows) on return, e = D^-1 U z.
+template <typename MT>
+void BsrSystem::red_apply_t(const MT* vals, const double* dinv, const double* src, double* z, double* e, double* out,
+                            bool second) {
+    const RedView R = red_view();
+    const int ng = groups_fwd();
+    auto pass = [&](int kind, int g, const PassCount& c, double vectors) {
+        ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, red_bytes(c, c.rows, vectors));
+        launch_red_sweep<MT>(R, vals, dinv, kind, fwd_off_[g], fwd_off_[g + 1], src, w_.p, z, e, ks_.p, second,
+                             stream_);
+    };
+    for (int g = 2; g < ng; ++g) pass(RED_FWD, g, red_fwd_[g], 3.0);
+    for (int g = ng - 2; g >= 1; --g) pass(RED_BACK, g, red_back_[g], 3.0);
+    pass(RED_BACK0, 0, red_back_[0], 1.0);
+    ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, red_bytes(red_lower_, 0.0, 3.0));
+    launch_red_product<MT>(R, vals, src, e, out, r0_.p, ks_.p, partials_.p, !second, stream_);
+}
+
+// One BiCGSTAB iteration (bicgstab.cpp:84-176); every kernel is gated by the
+// device-side state.  e of the first product lies in t (written by the
+// second), e of the second in r (rewritten by the update).
+template <typename MT>
+void BsrSystem::red_iteration_t(const MT* vals, const double* dinv, bool use_cond) {
+    const RedView R = red_view();
+    const double rest = double(n_ - R.n0) * bs_ * 8.0, c1 = double(R.n1 - R.n0) * bs_;
+    red_apply_t<MT>(vals, dinv, p_.p, phat_.p, t_.p, v_.p, false);
+    {
+        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 3.0 * rest + c1 * (bs_ * 8.0 + 16.0));
+        launch_red_s(R, dinv, r_.p, v_.p, w_.p, s_.p, shat_.p, ks_.p, stream_);
+    }
+    red_apply_t<MT>(vals, dinv, s_.p, shat_.p, r_.p, t_.p, true);
+    ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 10.0 * rest + c1 * (bs_ * 8.0 + 16.0));
+    launch_red_update(R, dinv, shat_.p, s_.p, t_.p, v_.p, w_.p, r_.p, p_.p, phat_.p, ks_.p, partials_.p, loop_handle_,
+                      use_cond, stream_);
+}
+
+// x on colour 0 from its own rows.
+template <typename MT>
+void BsrSystem::red_end_t(const MT* vals, const double* dinv) {
+    ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, red_bytes(red_back_[0], red_back_[0].rows, 3.0));
+    launch_red_sweep<MT>(red_view(), vals, dinv, RED_XRED, 0, fwd_off_[1], r0_.p, nullptr, nullptr, nullptr, ks_.p,
+                         false, stream_);
+}
+
+// The whole solve as one graph: [begin] -> while [iteration] -> [end].  An
+// error on the way leaves the host loop in charge.
+bool BsrSystem::red_graph_ready(Start start) {
+    if (red_exec_precision_ != precision_) release_red_graphs();
+    if (red_exec_[start]) return true;
+    if (loop_failed_) return false;
+    const bool mixed = precision_ == CFDG_PREC_MIXED;
+    const int64_t launches0 = prof_->launches;
+    cudaGraph_t g = nullptr;
+    bool capturing = false;
+    auto end_capture = [&] {
+        cudaGraph_t out = nullptr;
+        capturing = false;
+        cuda_check(cudaStreamEndCapture(stream_, &out), "graph capture end");
+    };
+    auto begin_capture = [&](cudaGraph_t into, const cudaGraphNode_t* deps, std::size_t n) {
+        cuda_check(cudaStreamBeginCaptureToGraph(stream_, into, deps, nullptr, n, cudaStreamCaptureModeThreadLocal),
+                   "graph capture");
+        capturing = true;
+    };
+    try {
+        cuda_check(cudaGraphCreate(&g, 0), "graph create");
+        cuda_check(cudaGraphConditionalHandleCreate(&loop_handle_, g, 0, cudaGraphCondAssignDefault), "graph handle");
+        begin_capture(g, nullptr, 0);
+        if (mixed) red_begin_t<float>(vals32_.p, dinv(), start);
+        else red_begin_t<double>(vals64_.p, dinv(), start);
+        launch_red_enter(ks_.p, loop_handle_, stream_);
+        ++prof_->launches;
+        cudaStreamCaptureStatus status;
+        const cudaGraphNode_t* deps = nullptr;
+        std::size_t ndeps = 0;
+        cuda_check(cudaStreamGetCaptureInfo(stream_, &status, nullptr, nullptr, &deps, &ndeps), "graph capture info");
+        const std::vector<cudaGraphNode_t> before(deps, deps + ndeps);
+        end_capture();
+        cudaGraphNodeParams cp{};
+        cp.type = cudaGraphNodeTypeConditional;
+        cp.conditional.handle = loop_handle_;
+        cp.conditional.type = cudaGraphCondTypeWhile;
+        cp.conditional.size = 1;
+        cudaGraphNode_t loop;
+        cuda_check(cudaGraphAddNode(&loop, g, before.data(), before.size(), &cp), "graph conditional node");
+        const int64_t l1 = prof_->launches;
+        begin_capture(cp.conditional.phGraph_out[0], nullptr, 0);
+        if (mixed) red_iteration_t<float>(vals32_.p, dinv(), true);
+        else red_iteration_t<double>(vals64_.p, dinv(), true);
+        end_capture();
+        red_body_launches_ = prof_->launches - l1;
+        begin_capture(g, &loop, 1);
+        if (mixed) red_end_t<float>(vals32_.p, dinv());
+        else red_end_t<double>(vals64_.p, dinv());
+        end_capture();
+        cuda_check(cudaGetLastError(), "graph capture");
+        cuda_check(cudaGraphInstantiate(&red_exec_[start], g, 0), "graph instantiate");
+    } catch (const Failure&) {
+        if (capturing) {
+            cudaGraph_t dead = nullptr;
+            cudaStreamEndCapture(stream_, &dead);
+        }
+        cudaGetLastError();
+        red_exec_[start] = nullptr;
+        loop_failed_ = true;
+    }
+    red_fixed_launches_[start] = prof_->launches - launches0 - red_body_launches_;
+    prof_->launches = launches0;
+    if (g) cudaGraphDestroy(g);
+    red_exec_precision_ = precision_;
+    return red_exec_[start] != nullptr;
+}
+
+void BsrSystem::release_red_graphs() {
+    for (cudaGraphExec_t& e : red_exec_) {
+        if (e) cudaGraphExecDestroy(e);
+        e = nullptr;
+    }
+}
+
+cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, int max_it, double* x, const double* b,
+                                               Start start) {
+    const bool mixed = precision_ == CFDG_PREC_MIXED;
+    *ks_init_ = KrylovScalars{};
+    ks_init_->max_it = max_it;
+    ks_init_->rel_tol = rel_tol;
+    ks_init_->abs_tol = abs_tol;
+    ks_init_->guess = start == START_GUESS ? 1 : 0;
+    ks_init_->x = x;
+    ks_init_->b = b;
+    cuda_check(cudaMemcpyAsync(ks_.p, ks_init_, sizeof(KrylovScalars), cudaMemcpyHostToDevice, stream_), "H2D");
+    if (start != START_ZERO) {
+        DotSpec none{};
+        ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, spmv_bytes(0, false));
+        if (mixed) launch_spmv_ex<float>(view(), vals32_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
+        else launch_spmv_ex<double>(view(), vals64_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
+    }
+    auto read = [&] {
+        cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_), "D2H");
+        cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
+    };
+    if (device_loop && !prof_->on() && red_graph_ready(start)) {
+        cuda_check(cudaGraphLaunch(red_exec_[start], stream_), "krylov graph launch");
+        read();
+        prof_->launches += red_fixed_launches_[start] + red_body_launches_ * ks_host_->body_runs;
+    } else {
+        if (mixed) red_begin_t<float>(vals32_.p, dinv(), start);
+        else red_begin_t<double>(vals64_.p, dinv(), start);
+        int it = 0;
+        bool done = false;
+        while (!done && it < max_it) {
+            if (mixed) red_iteration_t<float>(vals32_.p, dinv(), false);
+            else red_iteration_t<double>(vals64_.p, dinv(), false);
+            ++it;
+            if (it % check_every == 0 || it == max_it) {
+                read();
+                if (ks_host_->state != KS_RUNNING) done = true;
+            }
+        }
+        if (mixed) red_end_t<float>(vals32_.p, dinv());
+        else red_end_t<double>(vals64_.p, dinv());
+        cuda_check(cudaGetLastError(), "krylov launch");
+        read();
+    }
+    last_guess_ = start == START_GUESS ? ks_host_->guess : 0;
+    last_bnorm_ = ks_host_->bnorm;
+    return krylov_result();
+}
+
+// A state still running stopped at the iteration cap.
+cfdg_krylov_result BsrSystem::krylov_result() const {
+    cfdg_krylov_result res{};
+    switch (ks_host_->state) {
+        case KS_CONVERGED: res.status = CFDG_KRYLOV_CONVERGED; break;
+        case KS_DIVERGED: res.status = CFDG_KRYLOV_DIVERGED; break;
+        default: res.status = CFDG_KRYLOV_MAX_ITERATIONS; break;
+    }
+    res.iterations = ks_host_->it;
+    res.initial_residual = ks_host_->initial;
+    res.final_residual = ks_host_->rnorm;
+    return res;
+}
+
 cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_tol, int max_it, double* x,
-                                       const double* b, bool guess) {
+                                       const double* b, Start start) {
     if (precond == CFDG_PC_SGS && !lu_ready_) throw Failure{CFDG_ERR_INVALID, "SGS preconditioner not set up"};
     const int64_t N = int64_t(n_) * bs_;
+    if (precond == CFDG_PC_SGS && !product_ && reducible())
+        return bicgstab_reduced(rel_tol, abs_tol, max_it, x, b, start);
+    const bool guess = start == START_GUESS;
+    if (start == START_ZERO) cuda_check(cudaMemsetAsync(x, 0, sizeof(double) * N, stream_), "memset");
     const BsrView A = view();
     const bool mixed = precision_ == CFDG_PREC_MIXED;
     KrylovScalars init{};
@@ -805,17 +1140,7 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
     cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
     last_guess_ = guess ? ks_host_->guess : 0;
     last_bnorm_ = ks_host_->bnorm;
-    cfdg_krylov_result res{};
-    switch (ks_host_->state) {
-        case KS_CONVERGED: res.status = CFDG_KRYLOV_CONVERGED; break;
-        case KS_DIVERGED: res.status = CFDG_KRYLOV_DIVERGED; break;
-        default: res.status = CFDG_KRYLOV_MAX_ITERATIONS; break;
-    }
-    if (max_it <= 0 && ks_host_->state == KS_RUNNING) res.status = CFDG_KRYLOV_MAX_ITERATIONS;
-    res.iterations = ks_host_->it;
-    res.initial_residual = ks_host_->initial;
-    res.final_residual = ks_host_->rnorm;
-    return res;
+    return krylov_result();
 }
 
 void BsrSystem::gm_alloc(int restart) {
@@ -1384,6 +1709,16 @@ void Solver::setup_matrix(const HostMesh& hm, const Csr& c2c) {
     sys_ = std::make_unique<BsrSystem>(device_, n, nv_, row_ptr.data(), cols.data(),
                                        pre_freeze_phase() ? CFDG_PREC_FP64 : cfg_.precision, stream_);
     sys_->device_loop = cfg_.krylov_loop == CFDG_KRYLOV_DEVICE_LOOP;
+    // The reduced solve has the iterates of the full one up to rounding.  On
+    // the wall-stretched viscous systems an unconverged solve amplifies
+    // rounding up to 1e13 times (two solves whose input differs by one unit in
+    // the last place end 1e-3 apart on the Spalart-Allmaras plate, 30
+    // iterations), and its FP64 D^-1 is another preconditioner than the
+    // FP32-rounded one of a mixed-precision solve (the supersonic ramp moves by
+    // 1e-6 in three steps): there the full solve stays.  Inviscid FP64 solves
+    // agree to 1e-12, and are 1.2x faster (4,096-cell ramp, ten steady
+    // iterations: 2.91 -> 2.41 ms).
+    sys_->reduce = cfg_.viscous ? BsrSystem::REDUCE_NONE : BsrSystem::REDUCE_FP64;
     auto pos = [&](int32_t row, int32_t col) -> int32_t {
         const auto b = cols.begin() + row_ptr[row], e = cols.begin() + row_ptr[row + 1];
         const auto it = std::lower_bound(b, e, col);
@@ -1716,14 +2051,13 @@ cfdg_krylov_result Solver::linear_solve() {
     if (use_guess) {
         ProfScope ps(&prof_, CFDG_KCAT_GUESS, stream_, 1, double(dm_.n) * (kMlpIn * 2.0 + nv_ * 8.0));
         guess_->forward(feat_.p, dm_.n, gscale_.p + 8, du_.p, stream_);
-    } else {
-        cuda_check(cudaMemsetAsync(du_.p, 0, du_.count * sizeof(double), stream_), "memset");
     }
+    const BsrSystem::Start start = use_guess ? BsrSystem::START_GUESS : BsrSystem::START_ZERO;
     last_jf_ = last_fallback_ = false;
     last_used_guess_ = use_guess;
     if (!jf_now()) {
         last_krylov_ = sys_->bicgstab(cfg_.precond, cfg_.lin_rel_tol, cfg_.lin_abs_tol, cfg_.lin_max_iterations,
-                                      du_.p, b_.p, use_guess);
+                                      du_.p, b_.p, start);
         return last_krylov_;
     }
     // Jacobian-free solve, replaced by the Picard solve when it does not
@@ -1743,7 +2077,7 @@ cfdg_krylov_result Solver::linear_solve() {
                              du_.p, b_.p, use_guess);
         else
             kr = sys_->bicgstab(cfg_.precond, cfg_.jf_rel_tol, cfg_.lin_abs_tol, cfg_.jf_max_iterations, du_.p, b_.p,
-                                use_guess);
+                                start);
     } catch (...) {
         sys_->set_product(nullptr);
         throw;
@@ -1756,9 +2090,8 @@ cfdg_krylov_result Solver::linear_solve() {
         last_krylov_ = kr;
         return last_krylov_;
     }
-    cuda_check(cudaMemsetAsync(du_.p, 0, du_.count * sizeof(double), stream_), "memset");
     cfdg_krylov_result pk = sys_->bicgstab(cfg_.precond, cfg_.lin_rel_tol, cfg_.lin_abs_tol,
-                                           cfg_.lin_max_iterations, du_.p, b_.p, false);
+                                           cfg_.lin_max_iterations, du_.p, b_.p, BsrSystem::START_ZERO);
     pk.iterations += kr.iterations;
     last_fallback_ = true;
     last_used_guess_ = false;

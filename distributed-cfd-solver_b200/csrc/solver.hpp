@@ -162,11 +162,13 @@ public:
     // with the split multicolour sweep the product on colour 0 is fused into
     // its last pass.  Returns the number of partial rows written.
     int sgs_apply_spmv(const double* r, double* z, double* y, const DotSpec& ds, double* partials, const int* active);
-    // BiCGSTAB on device vectors; x holds the initial guess.
-    // guess: x holds an initial guess that is replaced by x = 0 when
-    // ||b - A x|| >= ||b||; last_guess() tells 1 accepted, 2 rejected.
+    // Starting vector of a solve: x as given; x as a guess that is replaced
+    // by x = 0 when ||b - A x|| >= ||b|| (last_guess() tells 1 accepted, 2
+    // rejected); or zero, whatever x holds.
+    enum Start { START_GIVEN = 0, START_GUESS = 1, START_ZERO = 2 };
+    // BiCGSTAB on device vectors.
     cfdg_krylov_result bicgstab(int precond, double rel_tol, double abs_tol, int max_it, double* x, const double* b,
-                                bool guess = false);
+                                Start start = START_GIVEN);
     // Restarted GMRES(restart), right-preconditioned, on the same operator
     // (the stored matrix or the matrix-free product); same conventions as
     // bicgstab.  The basis is allocated on first use.
@@ -187,9 +189,15 @@ public:
     void set_product(Product p) { product_ = std::move(p); }
     int check_every = 1;  // host loop: polls the Krylov state every k iterations
     bool device_loop = true;  // run the iterations as one graph launch (CFDG_KRYLOV_DEVICE_LOOP)
+    // Systems whose multicolour BiCGSTAB runs in its reduced form
+    // (kernels_reduced.cu).
+    enum Reduce { REDUCE_NONE, REDUCE_FP64, REDUCE_ANY };
+    Reduce reduce = REDUCE_ANY;
 
 private:
     void build_ordering(int ordering);
+    void count_pass_bytes();
+    bool bytes_counted_ = false;
     template <typename F>
     bool device_loop_ready(int precond, double* x, const double* b, F&& iteration);
     void release_device_loop();
@@ -197,6 +205,25 @@ private:
     void sgs_apply_t(const MT* vals, const MT* lu, const double* r, double* z, const int* active,
                      bool skip_last = false);
     bool fuse_last_spmv() const { return split_ && sweeps_ == 1 && groups_bwd() >= 2; }
+    // BiCGSTAB + one multicolour sweep on the rows outside the first colour
+    // (kernels_reduced.cu)
+    bool reducible() const {
+        return reducible_ && sweeps_ == 1 && (reduce == REDUCE_ANY || (reduce == REDUCE_FP64 && precision_ == CFDG_PREC_FP64));
+    }
+    cfdg_krylov_result bicgstab_reduced(double rel_tol, double abs_tol, int max_it, double* x, const double* b,
+                                        Start start);
+    template <typename MT>
+    void red_begin_t(const MT* vals, const double* dinv, Start start);
+    template <typename MT>
+    void red_iteration_t(const MT* vals, const double* dinv, bool use_cond);
+    template <typename MT>
+    void red_apply_t(const MT* vals, const double* dinv, const double* src, double* z, double* e, double* out,
+                     bool second);
+    template <typename MT>
+    void red_end_t(const MT* vals, const double* dinv);
+    bool red_graph_ready(Start start);
+    void release_red_graphs();
+    cfdg_krylov_result krylov_result() const;
 
     int device_;
     cudaStream_t stream_;
@@ -213,7 +240,7 @@ private:
     int last_guess_ = 0;
     double last_bnorm_ = 0.0;
     bool lu_ready_ = false;
-    std::vector<int32_t> fwd_off_, bwd_off_;
+    std::vector<int32_t> fwd_off_, bwd_off_, fwd_rows_h_, bwd_rows_h_;
     std::vector<int32_t> fwd_first_, bwd_first_;  // first row of a contiguous group, -1 otherwise
     // algorithmic bytes of one pass, mode 0 / 1 / split half: the part that
     // does not depend on the matrix precision, and the matrix blocks read
@@ -226,6 +253,26 @@ private:
     bool level_coop_ = true;                  // cleared when the cooperative launch is unavailable
     int level_cluster_ = 0, level_smem_ = 0;  // level sweep in one cluster: CTAs (0: not used), shared memory each
     double spmv_bytes(int n_extra_vectors, bool read_y) const;
+    // reduced BiCGSTAB: at least two colours, and the rows are in colour order
+    // or have two colours; blocks and distinct vector entries its passes read
+    bool reducible_ = false;
+    DevArray<int32_t> mid_;    // first block of a row outside the colour-0 columns
+    DevArray<double> w_, dinv64_;
+    struct PassCount {
+        double rows = 0.0, blocks = 0.0, entries = 0.0;
+    };
+    std::vector<PassCount> red_back_, red_fwd_;  // per colour
+    PassCount red_lower_, red_w_;
+    double red_bytes(const PassCount& c, double dinv_rows, double vectors) const;
+    RedView red_view() const;
+    const double* dinv() const { return precision_ == CFDG_PREC_MIXED ? dinv64_.p : lu64_.p; }
+    // [start]: initial residual and w, the iterations as a conditional
+    // while-node, and x on colour 0, on the system's own buffers (the
+    // caller's x and b are read through the device scalars)
+    cudaGraphExec_t red_exec_[3] = {nullptr, nullptr, nullptr};
+    int red_exec_precision_ = -1;
+    int64_t red_fixed_launches_[3] = {0, 0, 0}, red_body_launches_ = 0;
+    KrylovScalars* ks_init_ = nullptr;  // pinned: the scalars a solve starts from
     // rows [fwd_off_[1], n) of a colour-ordered matrix: block count and
     // distinct columns (the SpMV left after the fused colour-0 product)
     double rest_nnzb_ = 0.0, rest_cols_ = 0.0;
