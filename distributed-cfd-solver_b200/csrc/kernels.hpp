@@ -107,6 +107,10 @@ void launch_gm_dots(int64_t len, const double* V, int64_t ld, int k0, int kn, co
                     double* h, cudaStream_t s);
 void launch_gm_update(int64_t len, const double* V, int64_t ld, int kn, const double* h, double* w, bool subtract,
                       cudaStream_t s);
+// w -= sum h_k V_k with *norm2 = |w|^2 of the result; w /= sqrt(*norm2)
+void launch_gm_update_norm(int64_t len, const double* V, int64_t ld, int kn, const double* h, double* w,
+                           double* partials, double* norm2, cudaStream_t s);
+void launch_gm_normalise(int64_t len, const double* norm2, double* w, cudaStream_t s);
 void launch_gm_axpy(int64_t len, double a, const double* x, double* y, bool accumulate, cudaStream_t s);
 
 // ------------------------------------------------------------ linear algebra

@@ -270,6 +270,7 @@ BsrSystem::~BsrSystem() {
     if (ks_init_) cudaFreeHost(ks_init_);
     if (ks_host_) cudaFreeHost(ks_host_);
     if (gm_h_host_) cudaFreeHost(gm_h_host_);
+    if (gm_read_) cudaEventDestroy(gm_read_);
 }
 
 void BsrSystem::set_precision(int precision) {
@@ -1152,6 +1153,7 @@ void BsrSystem::gm_alloc(int restart) {
     alloc_or_throw(gm_part_, static_cast<std::size_t>(gm_partial_blocks(int64_t(N))) * gm_chunk() + 8, "GMRES partials");
     alloc_or_throw(gm_h_, 3 * static_cast<std::size_t>(restart + 1) + 8, "GMRES coefficients");
     cuda_check(cudaMemsetAsync(gm_h_.p, 0, gm_h_.count * sizeof(double), stream_), "memset");
+    if (!gm_read_) cuda_check(cudaEventCreateWithFlags(&gm_read_, cudaEventDisableTiming), "cudaEventCreate");
     if (gm_h_host_) cudaFreeHost(gm_h_host_);
     gm_h_host_ = nullptr;
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&gm_h_host_), sizeof(double) * (3 * (restart + 1) + 8)),
@@ -1257,9 +1259,9 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
         g[0] = beta;
         int k = 0;
         double resid = beta;
+        precond_apply(vec(0), gm_z_.p);
         for (int j = 0; j < m && its < max_it; ++j) {
             double* w = vec(j + 1);
-            precond_apply(vec(j), gm_z_.p);
             apply_A(gm_z_.p, w);
             dots(j + 1, w, hd);
             {
@@ -1268,11 +1270,20 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
             }
             dots(j + 1, w, hd + m + 1);
             {
-                ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 8.0 * N * (j + 3));
-                launch_gm_update(N, V, N, j + 1, hd + m + 1, w, true, stream_);
+                ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 2, 8.0 * N * (j + 3));
+                launch_gm_update_norm(N, V, N, j + 1, hd + m + 1, w, gm_part_.p, hd + 2 * m + 2, stream_);
             }
-            norm2(w, hd + 2 * m + 2);
-            read_h(2 * m + 3);
+            cuda_check(cudaMemcpyAsync(hh, hd, sizeof(double) * (2 * m + 3), cudaMemcpyDeviceToHost, stream_), "D2H");
+            cuda_check(cudaEventRecord(gm_read_, stream_), "event");
+            // the next basis vector and its preconditioner application run
+            // while the host reads the column (one application too many when
+            // it ends the cycle)
+            {
+                ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 8.0 * N * 2.0);
+                launch_gm_normalise(N, hd + 2 * m + 2, w, stream_);
+            }
+            if (j + 1 < m && its + 1 < max_it) precond_apply(w, gm_z_.p);
+            cuda_check(cudaEventSynchronize(gm_read_), "gmres sync");
             ++its;
             double col[201];
             for (int i = 0; i <= j; ++i) col[i] = hh[i] + hh[m + 1 + i];
@@ -1300,7 +1311,6 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
                 state = KS_CONVERGED;
                 break;
             }
-            axpy(1.0 / hn, w, w, false);
         }
         if (k > 0) {
             // y = R^-1 g, x += M^-1 (V y)

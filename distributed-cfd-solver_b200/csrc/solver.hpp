@@ -304,6 +304,7 @@ private:
     // device and pinned host coefficients (3 x (restart + 1) + 8)
     DevArray<double> gm_V_, gm_z_, gm_part_, gm_h_;
     double* gm_h_host_ = nullptr;
+    cudaEvent_t gm_read_ = nullptr;  // the column's coefficients are on the host
     int gm_restart_ = 0;
     void gm_alloc(int restart);
 };
