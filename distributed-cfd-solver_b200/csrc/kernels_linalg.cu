@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(256) k_sgs_level_coop(BsrView A, const MT* __r
 // cluster has the bandwidth for it: the levels of such a system hold a few
 // hundred rows.  The arithmetic of a row is k_sgs_level_coop's to the bit: one
 // lane group per off-diagonal block, the products subtracted in ascending
-// column order, the pivoted substitution.
+// column order, the pivoted substitution.  3.2 us a level on the same plate
+// (a sweep 0.96 -> 0.66 ms).
 constexpr int kClusterThreads = 512;
 constexpr int kClusterWarps = kClusterThreads / 32;
 
@@ -714,7 +715,7 @@ __global__ void __launch_bounds__(256, BS <= 5 ? 6 : 5) k_sgs_last_spmv(BsrView 
 }
 
 // ------------------------------------------------------ Krylov kernels
-// r = b - v, r0 = r, p = r; partial sums of |b|^2 and |r|^2.
+// r = b - v (v null: r = b), r0 = r, p = r; partial sums of |b|^2 and |r|^2.
 __global__ void __launch_bounds__(kVecThreads) k_krylov_init(int64_t len, const double* __restrict__ b,
                                                              const double* __restrict__ v, double* __restrict__ r,
                                                              double* __restrict__ r0, double* __restrict__ p,
@@ -723,7 +724,7 @@ __global__ void __launch_bounds__(kVecThreads) k_krylov_init(int64_t len, const 
     double pr[2] = {0.0, 0.0};
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < len; t += stride) {
         const double bt = b[t];
-        const double rt = bt + (-1.0) * v[t];
+        const double rt = v ? bt + (-1.0) * v[t] : bt;
         r[t] = rt;
         r0[t] = rt;
         p[t] = rt;

@@ -261,6 +261,7 @@ BsrSystem::BsrSystem(int device, int32_t n, int32_t bs, const int32_t* row_ptr, 
     alloc_or_throw(ks_, 1, "krylov scalars");
     alloc_or_throw(err_, 1, "error flag");
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_host_), sizeof(KrylovScalars)), "cudaMallocHost");
+    cuda_check(cudaMallocHost(reinterpret_cast<void**>(&err_host_), sizeof(int)), "cudaMallocHost");
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_init_), sizeof(KrylovScalars)), "cudaMallocHost");
 }
 
@@ -269,6 +270,7 @@ BsrSystem::~BsrSystem() {
     release_red_graphs();
     if (ks_init_) cudaFreeHost(ks_init_);
     if (ks_host_) cudaFreeHost(ks_host_);
+    if (err_host_) cudaFreeHost(err_host_);
     if (gm_h_host_) cudaFreeHost(gm_h_host_);
     if (gm_read_) cudaEventDestroy(gm_read_);
 }
@@ -593,7 +595,7 @@ void BsrSystem::count_pass_bytes() {
     bytes_counted_ = true;
 }
 
-void BsrSystem::sgs_setup(int ordering, int sweeps) {
+void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
     if (ordering != CFDG_SGS_LEVEL && ordering != CFDG_SGS_COLOR) throw Failure{CFDG_ERR_INVALID, "unknown SGS ordering"};
     if (sweeps < 1) throw Failure{CFDG_ERR_INVALID, "SGS sweeps must be >= 1"};
     if (ordering != ordering_) build_ordering(ordering);
@@ -616,16 +618,30 @@ void BsrSystem::sgs_setup(int ordering, int sweeps) {
         launch_lu_setup<double>(view(), vals64_.p, lu64_.p, nullptr, piv_.p, err_.p, color, stream_);
     }
     cuda_check(cudaGetLastError(), "lu launch");
-    int err = 0;
-    cuda_check(cudaMemcpyAsync(&err, err_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
-    cuda_check(cudaStreamSynchronize(stream_), "lu sync");
-    if (err > 0) {
-        throw Failure{CFDG_ERR_SINGULAR, "SgsPreconditioner: singular diagonal block at row " + std::to_string(err - 1)};
-    }
-    if (err < 0) {
-        throw Failure{CFDG_ERR_NONFINITE, "SgsPreconditioner: non-finite diagonal block at row " + std::to_string(-err - 1)};
-    }
     lu_ready_ = true;
+    lu_unchecked_ = true;
+    if (check) {
+        read_flag();
+        cuda_check(cudaStreamSynchronize(stream_), "lu sync");
+        check_factorisation();
+    }
+}
+
+// Queues the copy of the factorisation's flag, if nobody has read it yet.
+void BsrSystem::read_flag() {
+    if (lu_unchecked_)
+        cuda_check(cudaMemcpyAsync(err_host_, err_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
+}
+
+void BsrSystem::check_factorisation() {
+    if (!lu_unchecked_) return;
+    lu_unchecked_ = false;
+    const int err = *err_host_;
+    if (err == 0) return;
+    lu_ready_ = false;
+    if (err > 0)
+        throw Failure{CFDG_ERR_SINGULAR, "SgsPreconditioner: singular diagonal block at row " + std::to_string(err - 1)};
+    throw Failure{CFDG_ERR_NONFINITE, "SgsPreconditioner: non-finite diagonal block at row " + std::to_string(-err - 1)};
 }
 
 template <typename MT>
@@ -962,10 +978,7 @@ cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, i
         if (mixed) launch_spmv_ex<float>(view(), vals32_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
         else launch_spmv_ex<double>(view(), vals64_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
     }
-    auto read = [&] {
-        cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_), "D2H");
-        cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
-    };
+    auto read = [&] { read_scalars(); };
     if (device_loop && !prof_->on() && red_graph_ready(start)) {
         cuda_check(cudaGraphLaunch(red_exec_[start], stream_), "krylov graph launch");
         read();
@@ -994,6 +1007,14 @@ cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, i
     return krylov_result();
 }
 
+// The solve's scalars on the host, with the factorisation's verdict.
+void BsrSystem::read_scalars() {
+    cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_), "D2H");
+    read_flag();
+    cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
+    check_factorisation();
+}
+
 // A state still running stopped at the iteration cap.
 cfdg_krylov_result BsrSystem::krylov_result() const {
     cfdg_krylov_result res{};
@@ -1015,15 +1036,14 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
     if (precond == CFDG_PC_SGS && !product_ && reducible())
         return bicgstab_reduced(rel_tol, abs_tol, max_it, x, b, start);
     const bool guess = start == START_GUESS;
-    if (start == START_ZERO) cuda_check(cudaMemsetAsync(x, 0, sizeof(double) * N, stream_), "memset");
     const BsrView A = view();
     const bool mixed = precision_ == CFDG_PREC_MIXED;
-    KrylovScalars init{};
-    init.max_it = max_it;
-    init.rel_tol = rel_tol;
-    init.abs_tol = abs_tol;
-    init.guess = guess ? 1 : 0;
-    cuda_check(cudaMemcpyAsync(ks_.p, &init, sizeof(init), cudaMemcpyHostToDevice, stream_), "H2D");
+    *ks_init_ = KrylovScalars{};
+    ks_init_->max_it = max_it;
+    ks_init_->rel_tol = rel_tol;
+    ks_init_->abs_tol = abs_tol;
+    ks_init_->guess = guess ? 1 : 0;
+    cuda_check(cudaMemcpyAsync(ks_.p, ks_init_, sizeof(KrylovScalars), cudaMemcpyHostToDevice, stream_), "H2D");
     const int* active = &ks_.p->state;
     const bool matrix_free = static_cast<bool>(product_);
     // y = A x (or the matrix-free product) with the dots ds; returns the partial rows
@@ -1038,20 +1058,18 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
     {
         DotSpec none{};
         none.n = 0;
-        if (matrix_free) {
-            if (guess) {
-                product_(x, v_.p, none, nullptr, nullptr);
-            } else {  // x = 0: A x = 0 without a residual evaluation
-                ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 8.0 * N);
-                cuda_check(cudaMemsetAsync(v_.p, 0, sizeof(double) * N, stream_), "memset");
-            }
+        const bool zero = start == START_ZERO || (matrix_free && !guess);  // x = 0: r = b without a product
+        if (zero) {
+            cuda_check(cudaMemsetAsync(x, 0, sizeof(double) * N, stream_), "memset");
+        } else if (matrix_free) {
+            product_(x, v_.p, none, nullptr, nullptr);
         } else {
             ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, spmv_bytes(0, false));
             if (mixed) launch_spmv_ex<float>(A, vals32_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
             else launch_spmv_ex<double>(A, vals64_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
         }
-        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 2, 5.0 * 8.0 * N);
-        launch_krylov_init(N, b, v_.p, r_.p, r0_.p, p_.p, partials_.p, ks_.p, stream_);
+        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 2, (zero ? 4.0 : 5.0) * 8.0 * N);
+        launch_krylov_init(N, b, zero ? nullptr : v_.p, r_.p, r0_.p, p_.p, partials_.p, ks_.p, stream_);
         if (guess) {
             ++prof_->launches;
             launch_krylov_guess_reset(N, ks_.p, b, x, r_.p, r0_.p, p_.p, stream_);
@@ -1115,8 +1133,8 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
     };
     if (device_loop && !matrix_free && !prof_->on() && max_it > 0 && device_loop_ready(precond, x, b, iteration)) {
         cuda_check(cudaGraphLaunch(loop_exec_, stream_), "krylov graph launch");
-        cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_), "D2H");
-        cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
+        cuda_check(cudaGetLastError(), "krylov launch");
+        read_scalars();
         prof_->launches += loop_body_launches_ * ks_host_->body_runs;
     } else {
         int it = 0;
@@ -1125,20 +1143,13 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
             iteration();
             ++it;
             if (it % check_every == 0 || it == max_it) {
-                cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_),
-                           "D2H");
-                cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
+                read_scalars();
                 if (ks_host_->state != KS_RUNNING) done = true;
             }
         }
+        cuda_check(cudaGetLastError(), "krylov launch");
+        if (it == 0) read_scalars();
     }
-    {
-        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_);
-        launch_krylov_begin(ks_.p, stream_);  // marks max-iterations when still running
-    }
-    cuda_check(cudaGetLastError(), "krylov launch");
-    cuda_check(cudaMemcpyAsync(ks_host_, ks_.p, sizeof(KrylovScalars), cudaMemcpyDeviceToHost, stream_), "D2H");
-    cuda_check(cudaStreamSynchronize(stream_), "krylov sync");
     last_guess_ = guess ? ks_host_->guess : 0;
     last_bnorm_ = ks_host_->bnorm;
     return krylov_result();
@@ -1211,7 +1222,9 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
     };
     auto read_h = [&](int count) {
         cuda_check(cudaMemcpyAsync(hh, hd, sizeof(double) * count, cudaMemcpyDeviceToHost, stream_), "D2H");
+        read_flag();
         cuda_check(cudaStreamSynchronize(stream_), "gmres sync");
+        check_factorisation();
     };
     auto axpy = [&](double a, const double* xin, double* y, bool acc) {
         ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 8.0 * N * (acc ? 3.0 : 2.0));
@@ -2051,7 +2064,8 @@ void Solver::assemble_jacobian() {
 }
 
 cfdg_krylov_result Solver::linear_solve() {
-    if (cfg_.precond == CFDG_PC_SGS) sys_->sgs_setup(cfg_.sgs_ordering, std::max(cfg_.sgs_sweeps, 1));
+    // the factorisation's flag comes back with the solve's scalars
+    if (cfg_.precond == CFDG_PC_SGS) sys_->sgs_setup(cfg_.sgs_ordering, std::max(cfg_.sgs_sweeps, 1), false);
     const bool prefix = pre_freeze_phase();
     if ((guess_ && !prefix) || dataset_) prepare_guess_inputs();
     // the network predicts the update relative to the previous one: no

@@ -155,7 +155,9 @@ public:
     // y = alpha*A*x + beta*y (device vectors)
     void spmv(const double* x, double* y, double alpha, double beta);
     // SgsPreconditioner::setup: ordering + block LU of the diagonal.
-    void sgs_setup(int ordering, int sweeps);
+    // check: wait for the factorisation and throw on a singular or non-finite
+    // block; else the next solve reads the flag with its scalars and throws.
+    void sgs_setup(int ordering, int sweeps, bool check = true);
     // z = M^-1 r (device vectors).
     void sgs_apply(const double* r, double* z, const int* active);
     // z = M^-1 r, then y = A z with the dots `ds` (partials at `partials`);
@@ -224,6 +226,9 @@ private:
     bool red_graph_ready(Start start);
     void release_red_graphs();
     cfdg_krylov_result krylov_result() const;
+    void read_scalars();
+    void read_flag();
+    void check_factorisation();
 
     int device_;
     cudaStream_t stream_;
@@ -236,6 +241,8 @@ private:
     DevArray<float> vals32_, lu32_;
     DevArray<int8_t> piv_;
     DevArray<int> err_;
+    int* err_host_ = nullptr;   // pinned copy of the factorisation's flag
+    bool lu_unchecked_ = false; // ... which nobody has read yet
     int ordering_ = -1, sweeps_ = 1;
     int last_guess_ = 0;
     double last_bnorm_ = 0.0;
