@@ -1,6 +1,7 @@
 // Device-side data views and launch helpers shared by all kernels.
 #pragma once
 
+#include <cstddef>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -71,6 +72,39 @@ struct DevFields {
     double* rho;     // nt: density
     double* mut;     // nt: eddy viscosity
 };
+
+#ifdef __CUDACC__
+// Programmatic dependent launch.  A residual evaluation and a Jacobian-free
+// product are chains of kernels of 5 to 50 us; launched one after the other,
+// each pays the drain of its predecessor and its own start.  launch_after lets
+// a kernel's blocks become resident while the predecessor's last ones run, and
+// pdl_enter, the first statement of every kernel launched so, holds them there
+// until the predecessor has completed and its writes are visible; nothing is
+// read or written before it.  The parameters of such a kernel carry no
+// __restrict__ and what a predecessor writes is not read with __ldg: either
+// would let a load through the read-only path, which is for data that no
+// kernel in flight writes.  A predecessor launched in another way (a copy, a
+// cooperative launch, a caller's kernel) is waited for as usual.  A
+// Jacobian-free step of the 131k-cell plate (500 launches): 7.0 -> 6.2 ms.
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+void launch_after(void (*kernel)(P...), unsigned grid, unsigned block, std::size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+#endif
 
 inline unsigned grid_for(int64_t threads, int block) {
     const int64_t g = (threads + block - 1) / block;

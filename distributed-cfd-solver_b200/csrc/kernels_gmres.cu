@@ -29,9 +29,10 @@ inline unsigned gm_grid(int64_t len) {
 // pass and the host reading a column while the next product runs, a
 // Jacobian-free step of the 131k-cell plate takes 7.08 ms instead of 7.20.
 template <int C>
-__global__ void __launch_bounds__(kGmThreads) k_gm_dots(int64_t len, const double* __restrict__ V, int64_t ld, int k0,
-                                                        int kn, const double* __restrict__ w,
-                                                        double* __restrict__ partials) {
+__global__ void __launch_bounds__(kGmThreads) k_gm_dots(int64_t len, const double* V, int64_t ld, int k0,
+                                                        int kn, const double* w,
+                                                        double* partials) {
+    pdl_enter();
     double s[C];
 #pragma unroll
     for (int k = 0; k < C; ++k) s[k] = 0.0;
@@ -46,8 +47,9 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_dots(int64_t len, const doubl
 
 // h[k0 + k] = sum over blocks of partials[b * stride + k], one warp per
 // coefficient: lane-strided sums in block order, then a fixed shuffle tree.
-__global__ void k_gm_dots_fin(int nblocks, int stride, int k0, int kn, const double* __restrict__ partials,
-                              double* __restrict__ h) {
+__global__ void k_gm_dots_fin(int nblocks, int stride, int k0, int kn, const double* partials,
+                              double* h) {
+    pdl_enter();
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (k >= kn) return;
     double s = 0.0;
@@ -63,9 +65,10 @@ __global__ void k_gm_dots_fin(int nblocks, int stride, int k0, int kn, const dou
 // the new |w|^2 as k_gm_dots forms them.  Eight basis entries load at once; the
 // sum stays in order.
 template <bool SUBTRACT, bool NORM>
-__global__ void __launch_bounds__(kGmThreads) k_gm_update(int64_t len, const double* __restrict__ V, int64_t ld, int kn,
-                                                          const double* __restrict__ h, double* __restrict__ w,
-                                                          double* __restrict__ partials) {
+__global__ void __launch_bounds__(kGmThreads) k_gm_update(int64_t len, const double* V, int64_t ld, int kn,
+                                                          const double* h, double* w,
+                                                          double* partials) {
+    pdl_enter();
     constexpr int U = 8;
     double s[1] = {0.0};
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < len; t += int64_t(gridDim.x) * blockDim.x) {
@@ -89,16 +92,18 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_update(int64_t len, const dou
 }
 
 // w /= sqrt(*norm2): the basis vector of a Gram-Schmidt residual
-__global__ void __launch_bounds__(kGmThreads) k_gm_normalise(int64_t len, const double* __restrict__ norm2,
-                                                             double* __restrict__ w) {
+__global__ void __launch_bounds__(kGmThreads) k_gm_normalise(int64_t len, const double* norm2,
+                                                             double* w) {
+    pdl_enter();
     const double a = 1.0 / sqrt(fmax(*norm2, 0.0));
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < len; t += int64_t(gridDim.x) * blockDim.x)
         w[t] = a * w[t];
 }
 
 // y = a x (+ y when accumulate)
-__global__ void __launch_bounds__(kGmThreads) k_gm_axpy(int64_t len, double a, const double* __restrict__ x,
-                                                        double* __restrict__ y, int accumulate) {
+__global__ void __launch_bounds__(kGmThreads) k_gm_axpy(int64_t len, double a, const double* x,
+                                                        double* y, int accumulate) {
+    pdl_enter();
     for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < len; t += int64_t(gridDim.x) * blockDim.x)
         y[t] = accumulate ? y[t] + a * x[t] : a * x[t];
 }
@@ -114,33 +119,33 @@ void launch_gm_dots(int64_t len, const double* V, int64_t ld, int k0, int kn, co
     for (int c = 0; c < kn; c += kGmChunk) {
         const int m = kn - c < kGmChunk ? kn - c : kGmChunk;
         const int stride = m == 1 ? 1 : m <= 8 ? 8 : m <= 16 ? 16 : 24;
-        if (m == 1) k_gm_dots<1><<<gr, kGmThreads, 0, s>>>(len, V, ld, k0 + c, m, w, partials);
-        else if (m <= 8) k_gm_dots<8><<<gr, kGmThreads, 0, s>>>(len, V, ld, k0 + c, m, w, partials);
-        else if (m <= 16) k_gm_dots<16><<<gr, kGmThreads, 0, s>>>(len, V, ld, k0 + c, m, w, partials);
-        else k_gm_dots<24><<<gr, kGmThreads, 0, s>>>(len, V, ld, k0 + c, m, w, partials);
-        k_gm_dots_fin<<<1, 32 * m, 0, s>>>(static_cast<int>(gr), stride, k0 + c, m, partials, h);
+        if (m == 1) launch_after(k_gm_dots<1>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);
+        else if (m <= 8) launch_after(k_gm_dots<8>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);
+        else if (m <= 16) launch_after(k_gm_dots<16>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);
+        else launch_after(k_gm_dots<24>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);
+        launch_after(k_gm_dots_fin, 1, 32 * m, 0, s, static_cast<int>(gr), stride, k0 + c, m, partials, h);
     }
 }
 
 void launch_gm_update(int64_t len, const double* V, int64_t ld, int kn, const double* h, double* w, bool subtract,
                       cudaStream_t s) {
-    if (subtract) k_gm_update<true, false><<<gm_grid(len), kGmThreads, 0, s>>>(len, V, ld, kn, h, w, nullptr);
-    else k_gm_update<false, false><<<gm_grid(len), kGmThreads, 0, s>>>(len, V, ld, kn, h, w, nullptr);
+    if (subtract) launch_after(k_gm_update<true, false>, gm_grid(len), kGmThreads, 0, s, len, V, ld, kn, h, w, nullptr);
+    else launch_after(k_gm_update<false, false>, gm_grid(len), kGmThreads, 0, s, len, V, ld, kn, h, w, nullptr);
 }
 
 void launch_gm_update_norm(int64_t len, const double* V, int64_t ld, int kn, const double* h, double* w,
                            double* partials, double* norm2, cudaStream_t s) {
     const unsigned gr = gm_grid(len);
-    k_gm_update<true, true><<<gr, kGmThreads, 0, s>>>(len, V, ld, kn, h, w, partials);
-    k_gm_dots_fin<<<1, 32, 0, s>>>(static_cast<int>(gr), 1, 0, 1, partials, norm2);
+    launch_after(k_gm_update<true, true>, gr, kGmThreads, 0, s, len, V, ld, kn, h, w, partials);
+    launch_after(k_gm_dots_fin, 1, 32, 0, s, static_cast<int>(gr), 1, 0, 1, partials, norm2);
 }
 
 void launch_gm_normalise(int64_t len, const double* norm2, double* w, cudaStream_t s) {
-    k_gm_normalise<<<gm_grid(len), kGmThreads, 0, s>>>(len, norm2, w);
+    launch_after(k_gm_normalise, gm_grid(len), kGmThreads, 0, s, len, norm2, w);
 }
 
 void launch_gm_axpy(int64_t len, double a, const double* x, double* y, bool accumulate, cudaStream_t s) {
-    k_gm_axpy<<<gm_grid(len), kGmThreads, 0, s>>>(len, a, x, y, accumulate ? 1 : 0);
+    launch_after(k_gm_axpy, gm_grid(len), kGmThreads, 0, s, len, a, x, y, accumulate ? 1 : 0);
 }
 
 }  // namespace cfdg

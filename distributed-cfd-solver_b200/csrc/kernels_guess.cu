@@ -26,12 +26,13 @@ namespace {
 constexpr int kSumThreads = 256;
 
 template <int NV>
-__global__ void __launch_bounds__(kSumThreads) k_guess_sums(int32_t n, const int32_t* __restrict__ row_of,
-                                                           const double* __restrict__ b,
-                                                           const double* __restrict__ dt,
-                                                           const double* __restrict__ vol,
-                                                           const double* __restrict__ du_prev,
-                                                           double* __restrict__ partials) {
+__global__ void __launch_bounds__(kSumThreads) k_guess_sums(int32_t n, const int32_t* row_of,
+                                                           const double* b,
+                                                           const double* dt,
+                                                           const double* vol,
+                                                           const double* du_prev,
+                                                           double* partials) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     double acc[2 * NV];
 #pragma unroll
@@ -55,7 +56,8 @@ __global__ void __launch_bounds__(kSumThreads) k_guess_sums(int32_t n, const int
 // component that stays at round-off (spanwise momentum of a quasi-2-D flow)
 // is not blown up to O(1).
 template <int NV>
-__global__ void k_guess_scales(int32_t n, const double* __restrict__ partials, int nblocks, double* gscale) {
+__global__ void k_guess_scales(int32_t n, const double* partials, int nblocks, double* gscale) {
+    pdl_enter();
     __shared__ double sq[2 * NV];
     const int k = threadIdx.x;
     if (k < 2 * NV) {
@@ -77,11 +79,12 @@ __device__ __forceinline__ uint16_t bf(double x) {
 }
 
 template <int NV>
-__global__ void __launch_bounds__(128) k_guess_features(DevMesh m, const double* __restrict__ U,
-                                                       const double* __restrict__ b, const double* __restrict__ dt,
-                                                       const double* __restrict__ du_prev,
-                                                       const double* __restrict__ gscale, double lcfl,
-                                                       uint16_t* __restrict__ feat) {
+__global__ void __launch_bounds__(128) k_guess_features(DevMesh m, const double* U,
+                                                       const double* b, const double* dt,
+                                                       const double* du_prev,
+                                                       const double* gscale, double lcfl,
+                                                       uint16_t* feat) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
     const int64_t n = m.n;
@@ -150,9 +153,10 @@ __global__ void __launch_bounds__(128) k_guess_features(DevMesh m, const double*
 }
 
 // Samples c = phase + k * stride: features row and target dU / s_d.
-__global__ void k_guess_append(int32_t n, const int32_t* __restrict__ row_of, int nv, int32_t stride, int32_t phase,
-                               int64_t count, const uint16_t* __restrict__ feat, const double* __restrict__ du,
-                               const double* __restrict__ gscale, uint16_t* __restrict__ X, float* __restrict__ T) {
+__global__ void k_guess_append(int32_t n, const int32_t* row_of, int nv, int32_t stride, int32_t phase,
+                               int64_t count, const uint16_t* feat, const double* du,
+                               const double* gscale, uint16_t* X, float* T) {
+    pdl_enter();
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= count) return;
     const int64_t c0 = phase + k * stride;
@@ -173,11 +177,11 @@ void launch_guess_scales(int32_t n, const int32_t* row_of, int nv, const double*
                          const double* vol, const double* du_prev, double* partials, double* gscale, cudaStream_t s) {
     const int nb = guess_sum_blocks(n);
     if (nv == 6) {
-        k_guess_sums<6><<<nb, kSumThreads, 0, s>>>(n, row_of, b, dt, vol, du_prev, partials);
-        k_guess_scales<6><<<1, 32, 0, s>>>(n, partials, nb, gscale);
+        launch_after(k_guess_sums<6>, nb, kSumThreads, 0, s, n, row_of, b, dt, vol, du_prev, partials);
+        launch_after(k_guess_scales<6>, 1, 32, 0, s, n, partials, nb, gscale);
     } else {
-        k_guess_sums<5><<<nb, kSumThreads, 0, s>>>(n, row_of, b, dt, vol, du_prev, partials);
-        k_guess_scales<5><<<1, 32, 0, s>>>(n, partials, nb, gscale);
+        launch_after(k_guess_sums<5>, nb, kSumThreads, 0, s, n, row_of, b, dt, vol, du_prev, partials);
+        launch_after(k_guess_scales<5>, 1, 32, 0, s, n, partials, nb, gscale);
     }
 }
 
@@ -185,15 +189,16 @@ void launch_guess_features(const DevMesh& m, int nv, const double* U, const doub
                            const double* du_prev, const double* gscale, double cfl, uint16_t* feat, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, 128);
     const double lcfl = 0.25 * std::log10(cfl > 0.0 ? cfl : 1.0);
-    if (nv == 6) k_guess_features<6><<<gr, 128, 0, s>>>(m, U, b, dt, du_prev, gscale, lcfl, feat);
-    else k_guess_features<5><<<gr, 128, 0, s>>>(m, U, b, dt, du_prev, gscale, lcfl, feat);
+    if (nv == 6) launch_after(k_guess_features<6>, gr, 128, 0, s, m, U, b, dt, du_prev, gscale, lcfl, feat);
+    else launch_after(k_guess_features<5>, gr, 128, 0, s, m, U, b, dt, du_prev, gscale, lcfl, feat);
 }
 
 void launch_guess_append(int32_t n, const int32_t* row_of, int nv, int32_t stride, int32_t phase, int64_t count,
                          const uint16_t* feat, const double* du, const double* gscale, uint16_t* X, float* T,
                          cudaStream_t s) {
     if (count <= 0) return;
-    k_guess_append<<<grid_for(count, 128), 128, 0, s>>>(n, row_of, nv, stride, phase, count, feat, du, gscale, X, T);
+    launch_after(k_guess_append, grid_for(count, 128), 128, 0, s, n, row_of, nv, stride, phase, count, feat, du, gscale,
+                 X, T);
 }
 
 }  // namespace cfdg

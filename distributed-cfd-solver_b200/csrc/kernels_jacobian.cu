@@ -158,6 +158,7 @@ __device__ __forceinline__ double visc_entry(const ViscFace& v, const GasParams&
 template <typename MT, bool VISC, int BS, bool FULL>
 __global__ void __launch_bounds__(128, VISC ? 3 : 4)
     k_jac_rows(DevMesh m, DevFields f, GasParams g, JacStructure js, MT* vals) {
+    pdl_enter();
     __shared__ MT stage_all[4][32][stage_stride<BS>()];
     MT(*stage)[stage_stride<BS>()] = stage_all[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -296,11 +297,11 @@ static void launch_jacobian_t(const DevMesh& m, const DevFields& f, const GasPar
                               bool visc, MT* values, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, 128);
     if (bs == 5) {
-        if (visc) k_jac_rows<MT, true, 5, FULL><<<gr, 128, 0, s>>>(m, f, g, js, values);
-        else k_jac_rows<MT, false, 5, FULL><<<gr, 128, 0, s>>>(m, f, g, js, values);
+        if (visc) launch_after(k_jac_rows<MT, true, 5, FULL>, gr, 128, 0, s, m, f, g, js, values);
+        else launch_after(k_jac_rows<MT, false, 5, FULL>, gr, 128, 0, s, m, f, g, js, values);
     } else {
-        if (visc) k_jac_rows<MT, true, 6, FULL><<<gr, 128, 0, s>>>(m, f, g, js, values);
-        else k_jac_rows<MT, false, 6, FULL><<<gr, 128, 0, s>>>(m, f, g, js, values);
+        if (visc) launch_after(k_jac_rows<MT, true, 6, FULL>, gr, 128, 0, s, m, f, g, js, values);
+        else launch_after(k_jac_rows<MT, false, 6, FULL>, gr, 128, 0, s, m, f, g, js, values);
     }
 }
 

@@ -58,8 +58,9 @@ __device__ __forceinline__ void block_max_store(double (&val)[K], double* __rest
 
 // Per-block sums of U_v^2 (RMS of each conserved variable).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_sumsq(int32_t n, const double* __restrict__ U,
-                                                         double* __restrict__ partials) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_sumsq(int32_t n, const double* U,
+                                                         double* partials) {
+    pdl_enter();
     double s[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = 0.0;
@@ -75,8 +76,9 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_sumsq(int32_t n, const double
 // scal[v] = sqrt(mean U_v^2) + 1e-300: one block sums each variable's
 // partials (thread t: blocks t, t+T, ..., then the fixed-order tree).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_rms_fin(int nblocks, int32_t n, const double* __restrict__ partials,
-                                                           double* __restrict__ scal) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_rms_fin(int nblocks, int32_t n, const double* partials,
+                                                           double* scal) {
+    pdl_enter();
     __shared__ double tot[NV];
     double s[NV];
 #pragma unroll
@@ -91,8 +93,9 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_rms_fin(int nblocks, int32_t 
 
 // Per-block max |x_v| over the rows (x: AoS rows of NV).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_vmax(int32_t rows, const double* __restrict__ x,
-                                                        double* __restrict__ partials, const int* __restrict__ active) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_vmax(int32_t rows, const double* x,
+                                                        double* partials, const int* active) {
+    pdl_enter();
     if (active && *active != 0) return;
     double m[NV];
 #pragma unroll
@@ -105,9 +108,10 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_vmax(int32_t rows, const doub
 
 // eps = eps_rel / max_v(max|x_v| / rms(U_v)), 0 for x = 0 (scal[kJfEps]).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_eps(int nblocks, const double* __restrict__ partials,
-                                                       double* __restrict__ scal, double eps_rel,
-                                                       const int* __restrict__ active) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_eps(int nblocks, const double* partials,
+                                                       double* scal, double eps_rel,
+                                                       const int* active) {
+    pdl_enter();
     if (active && *active != 0) return;
     __shared__ double mx[NV];
     double m[NV];
@@ -127,10 +131,11 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_eps(int nblocks, const double
 
 // Up = U + eps x (x in row order).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_perturb(DevMesh m, const double* __restrict__ U,
-                                                           const double* __restrict__ x,
-                                                           const double* __restrict__ scal, double* __restrict__ Up,
-                                                           const int* __restrict__ active) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_perturb(DevMesh m, const double* U,
+                                                           const double* x,
+                                                           const double* scal, double* Up,
+                                                           const int* active) {
+    pdl_enter();
     if (active && *active != 0) return;
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
@@ -145,12 +150,13 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_perturb(DevMesh m, const doub
 // alpha - V diag is V/dt of the pseudo-time step alone: the BDF term of an
 // unsteady residual is inside R and its derivative inside the difference.
 template <int NV, int ND>
-__global__ void __launch_bounds__(kJfThreads) k_jf_combine(DevMesh m, const double* __restrict__ alpha, double diag,
-                                                           const double* __restrict__ x, const double* __restrict__ b,
-                                                           const double* __restrict__ resp,
-                                                           const double* __restrict__ scal, double* __restrict__ y,
-                                                           DotSpec ds, double* __restrict__ partials,
-                                                           const int* __restrict__ active) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_combine(DevMesh m, const double* alpha, double diag,
+                                                           const double* x, const double* b,
+                                                           const double* resp,
+                                                           const double* scal, double* y,
+                                                           DotSpec ds, double* partials,
+                                                           const int* active) {
+    pdl_enter();
     if (active && *active != 0) return;
     const double e = scal[kJfEps];
     const int64_t n = m.n;
@@ -183,10 +189,11 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_combine(DevMesh m, const doub
 // |du_E / E| and, with the turbulence variable, |du_nu| / (|rho nu~| +
 // 1e-3 rms(rho nu~)).
 template <int NV>
-__global__ void __launch_bounds__(kJfThreads) k_jf_step_ratio(DevMesh m, const double* __restrict__ U,
-                                                              const double* __restrict__ du,
-                                                              const double* __restrict__ scal,
-                                                              double* __restrict__ partials) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_step_ratio(DevMesh m, const double* U,
+                                                              const double* du,
+                                                              const double* scal,
+                                                              double* partials) {
+    pdl_enter();
     double w[1] = {0.0};
     const int64_t n = m.n;
     const double floor_nu = NV == 6 ? 1e-3 * scal[5] : 0.0;
@@ -200,8 +207,9 @@ __global__ void __launch_bounds__(kJfThreads) k_jf_step_ratio(DevMesh m, const d
 }
 
 // scal[kJfStep] = min(1, max_change / worst).
-__global__ void __launch_bounds__(kJfThreads) k_jf_step_fin(int nblocks, const double* __restrict__ partials,
-                                                            double max_change, double* __restrict__ scal) {
+__global__ void __launch_bounds__(kJfThreads) k_jf_step_fin(int nblocks, const double* partials,
+                                                            double max_change, double* scal) {
+    pdl_enter();
     __shared__ double mx[1];
     double w[1] = {0.0};
     for (int b = threadIdx.x; b < nblocks; b += blockDim.x) w[0] = fmax(w[0], partials[b]);
@@ -216,26 +224,26 @@ int jf_partial_blocks(int32_t n) { return static_cast<int>(jf_grid(n)); }
 
 void launch_jf_rms(int32_t n, int nv, const double* U, double* partials, double* scal, cudaStream_t s) {
     const unsigned gr = jf_grid(n);
-    if (nv == 6) k_jf_sumsq<6><<<gr, kJfThreads, 0, s>>>(n, U, partials);
-    else k_jf_sumsq<5><<<gr, kJfThreads, 0, s>>>(n, U, partials);
-    if (nv == 6) k_jf_rms_fin<6><<<1, kJfThreads, 0, s>>>(static_cast<int>(gr), n, partials, scal);
-    else k_jf_rms_fin<5><<<1, kJfThreads, 0, s>>>(static_cast<int>(gr), n, partials, scal);
+    if (nv == 6) launch_after(k_jf_sumsq<6>, gr, kJfThreads, 0, s, n, U, partials);
+    else launch_after(k_jf_sumsq<5>, gr, kJfThreads, 0, s, n, U, partials);
+    if (nv == 6) launch_after(k_jf_rms_fin<6>, 1, kJfThreads, 0, s, static_cast<int>(gr), n, partials, scal);
+    else launch_after(k_jf_rms_fin<5>, 1, kJfThreads, 0, s, static_cast<int>(gr), n, partials, scal);
 }
 
 void launch_jf_eps(int32_t rows, int nv, const double* x, double* partials, double* scal, double eps_rel,
                    const int* active, cudaStream_t s) {
     const unsigned gr = jf_grid(rows);
-    if (nv == 6) k_jf_vmax<6><<<gr, kJfThreads, 0, s>>>(rows, x, partials, active);
-    else k_jf_vmax<5><<<gr, kJfThreads, 0, s>>>(rows, x, partials, active);
-    if (nv == 6) k_jf_eps<6><<<1, kJfThreads, 0, s>>>(static_cast<int>(gr), partials, scal, eps_rel, active);
-    else k_jf_eps<5><<<1, kJfThreads, 0, s>>>(static_cast<int>(gr), partials, scal, eps_rel, active);
+    if (nv == 6) launch_after(k_jf_vmax<6>, gr, kJfThreads, 0, s, rows, x, partials, active);
+    else launch_after(k_jf_vmax<5>, gr, kJfThreads, 0, s, rows, x, partials, active);
+    if (nv == 6) launch_after(k_jf_eps<6>, 1, kJfThreads, 0, s, static_cast<int>(gr), partials, scal, eps_rel, active);
+    else launch_after(k_jf_eps<5>, 1, kJfThreads, 0, s, static_cast<int>(gr), partials, scal, eps_rel, active);
 }
 
 void launch_jf_perturb(const DevMesh& m, int nv, const double* U, const double* x, const double* scal, double* Up,
                        const int* active, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, kJfThreads);
-    if (nv == 6) k_jf_perturb<6><<<gr, kJfThreads, 0, s>>>(m, U, x, scal, Up, active);
-    else k_jf_perturb<5><<<gr, kJfThreads, 0, s>>>(m, U, x, scal, Up, active);
+    if (nv == 6) launch_after(k_jf_perturb<6>, gr, kJfThreads, 0, s, m, U, x, scal, Up, active);
+    else launch_after(k_jf_perturb<5>, gr, kJfThreads, 0, s, m, U, x, scal, Up, active);
 }
 
 int launch_jf_combine(const DevMesh& m, int nv, const double* alpha, double diag, const double* x, const double* b,
@@ -243,7 +251,7 @@ int launch_jf_combine(const DevMesh& m, int nv, const double* alpha, double diag
                       const int* active, cudaStream_t s) {
     const unsigned gr = jf_grid(m.n);
 #define CFDG_JFC(NV, ND) \
-    k_jf_combine<NV, ND><<<gr, kJfThreads, 0, s>>>(m, alpha, diag, x, b, resp, scal, y, ds, partials, active)
+    launch_after(k_jf_combine<NV, ND>, gr, kJfThreads, 0, s, m, alpha, diag, x, b, resp, scal, y, ds, partials, active)
     if (nv == 6) {
         if (ds.n == 0) CFDG_JFC(6, 0);
         else if (ds.n == 1) CFDG_JFC(6, 1);
@@ -260,9 +268,9 @@ int launch_jf_combine(const DevMesh& m, int nv, const double* alpha, double diag
 void launch_jf_step_scale(const DevMesh& m, int nv, const double* U, const double* du, double* partials, double* scal,
                           double max_change, cudaStream_t s) {
     const unsigned gr = jf_grid(m.n);
-    if (nv == 6) k_jf_step_ratio<6><<<gr, kJfThreads, 0, s>>>(m, U, du, scal, partials);
-    else k_jf_step_ratio<5><<<gr, kJfThreads, 0, s>>>(m, U, du, scal, partials);
-    k_jf_step_fin<<<1, kJfThreads, 0, s>>>(static_cast<int>(gr), partials, max_change, scal);
+    if (nv == 6) launch_after(k_jf_step_ratio<6>, gr, kJfThreads, 0, s, m, U, du, scal, partials);
+    else launch_after(k_jf_step_ratio<5>, gr, kJfThreads, 0, s, m, U, du, scal, partials);
+    launch_after(k_jf_step_fin, 1, kJfThreads, 0, s, static_cast<int>(gr), partials, max_change, scal);
 }
 
 }  // namespace cfdg

@@ -176,9 +176,10 @@ constexpr int kLuThreads = 128;
 // Occupancy bound per block size: the 6x6 factor, pivots and inverse
 // column of a thread spill below ~170 registers, the 5x5 ones below ~128.
 template <typename MT, int BS, bool INV>
-__global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, const MT* __restrict__ vals, MT* __restrict__ lu,
-                                                   double* __restrict__ inv64, int8_t* __restrict__ piv,
-                                                   int* __restrict__ err) {
+__global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, const MT* vals, MT* lu,
+                                                   double* inv64, int8_t* piv,
+                                                   int* err) {
+    pdl_enter();
     constexpr int B2 = BS * BS;
     constexpr int SP = B2 % 2 == 0 ? B2 + 1 : B2;  // odd row stride: thread-per-row accesses hit distinct banks
     __shared__ double sm[kLuThreads * SP];
@@ -990,8 +991,8 @@ void launch_lu_setup(const BsrView& A, const MT* vals, MT* lu, double* inv64, in
                      bool inverse, cudaStream_t s) {
     const unsigned gr = grid_for(A.n, kLuThreads);
 #define CFDG_LU(BS)                                                                          \
-    if (inverse) k_lu<MT, BS, true><<<gr, kLuThreads, 0, s>>>(A, vals, lu, inv64, piv, err_flag); \
-    else k_lu<MT, BS, false><<<gr, kLuThreads, 0, s>>>(A, vals, lu, inv64, piv, err_flag)
+    if (inverse) launch_after(k_lu<MT, BS, true>, gr, kLuThreads, 0, s, A, vals, lu, inv64, piv, err_flag); \
+    else launch_after(k_lu<MT, BS, false>, gr, kLuThreads, 0, s, A, vals, lu, inv64, piv, err_flag)
     switch (A.bs) {
         case 1: CFDG_LU(1); break;
         case 3: CFDG_LU(3); break;

@@ -18,6 +18,7 @@ namespace {
 // boundary faces (the owner primitive is recomputed from U with the same
 // arithmetic, so ghost and cell values agree bit for bit).
 __global__ void k_primitives(DevMesh m, DevFields f, GasParams g) {
+    pdl_enter();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t n = m.n, nt = m.nt;
     if (t < n) {
@@ -49,7 +50,8 @@ __global__ void k_primitives(DevMesh m, DevFields f, GasParams g) {
 // src/numerics/gradient/gradient_operator.cpp:340-391,549-599).
 // NVG variables starting at src (stride nt), written to dst planes.
 template <int NVG>
-__global__ void __launch_bounds__(128) k_gradient(DevMesh m, const double* __restrict__ src, double* __restrict__ dst) {
+__global__ void __launch_bounds__(128) k_gradient(DevMesh m, const double* src, double* dst) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t slice = c >> 5;
     if (int64_t(slice) * 32 >= m.n) return;  // whole warps only
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(128) k_gradient(DevMesh m, const double* __res
 // [n, n+nb) ghosts.
 template <bool LIMIT, int LIM>
 __global__ void __launch_bounds__(128) k_limiter_ghostgrad(DevMesh m, DevFields f, GasParams g, double k3) {
+    pdl_enter();
     // without the limiter (frozen or first order) the grid covers the ghosts only
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + (LIMIT ? 0 : int64_t(m.n));
     const int64_t n = m.n, nt = m.nt;
@@ -159,6 +162,7 @@ __global__ void __launch_bounds__(128) k_limiter_ghostgrad(DevMesh m, DevFields 
 // F (5) and A*s_max (+ viscous radius) for the cell gather.
 template <bool MUSCL, bool VISC>
 __global__ void __launch_bounds__(128, VISC ? 0 : 6) k_face_flux(DevMesh m, DevFields f, GasParams g) {
+    pdl_enter();
     const int32_t fc = blockIdx.x * blockDim.x + threadIdx.x;
     if (fc >= m.nf) return;
     const int64_t nt = m.nt;
@@ -224,6 +228,7 @@ __global__ void __launch_bounds__(128, VISC ? 0 : 6) k_face_flux(DevMesh m, DevF
 
 // Cell gather of face fluxes into R and lam (ascending face order).
 __global__ void __launch_bounds__(256) k_cell_residual(DevMesh m, DevFields f) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
     const int64_t n = m.n;
@@ -233,7 +238,7 @@ __global__ void __launch_bounds__(256) k_cell_residual(DevMesh m, DevFields f) {
         const int32_t es = __ldg(m.c2fs + e);  // the side is in the sign: no owner gather
         const int32_t fc = es >= 0 ? es : ~es;
         const double2* rec = reinterpret_cast<const double2*>(f.fflux + int64_t(fc) * 6);
-        const double2 a = __ldg(rec), b = __ldg(rec + 1), d = __ldg(rec + 2);
+        const double2 a = rec[0], b = rec[1], d = rec[2];
         const double F[5] = {a.x, a.y, b.x, b.y, d.x};
         if (es >= 0) {
 #pragma unroll
@@ -252,7 +257,8 @@ __global__ void __launch_bounds__(256) k_cell_residual(DevMesh m, DevFields f) {
 // Per-block partial sums of R_v^2 over cells (Solver::residual_norms,
 // solver.hpp:740-756); summed in fixed order by finalize_norms.
 template <int NV>
-__global__ void __launch_bounds__(256) k_norm_partials(int32_t n, const double* __restrict__ res, double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) k_norm_partials(int32_t n, const double* res, double* partials) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     double sq[NV];
 #pragma unroll
@@ -265,8 +271,9 @@ __global__ void __launch_bounds__(256) k_norm_partials(int32_t n, const double* 
 
 // Warp v sums column v of the partials (lane-strided, then a fixed shuffle
 // tree): deterministic for a given block count.
-__global__ void k_norm_finalize(int nblocks, int nv, const double* __restrict__ partials, double scale,
-                                double* __restrict__ l2) {
+__global__ void k_norm_finalize(int nblocks, int nv, const double* partials, double scale,
+                                double* l2) {
+    pdl_enter();
     const int v = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (v >= nv) return;
     double s = 0.0;
@@ -282,7 +289,8 @@ __global__ void k_norm_finalize(int nblocks, int nv, const double* __restrict__ 
 // the linear solve itself.  A 6-variable row of b is 48 bytes and stores as
 // three 16-byte pairs.
 template <int NV>
-__global__ void k_dt_rhs(DevMesh m, DevFields f, double cfl, double diag, double* __restrict__ b) {
+__global__ void k_dt_rhs(DevMesh m, DevFields f, double cfl, double diag, double* b) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
     const int64_t n = m.n;
@@ -310,8 +318,9 @@ __global__ void k_dt_rhs(DevMesh m, DevFields f, double cfl, double diag, double
 // (SpalartAllmaras::post_stage).  `scale` (device scalar, may be null):
 // U <- U + scale * du, the relaxed Jacobian-free step.
 template <int NV>
-__global__ void k_state_update(DevMesh m, double* __restrict__ U, const double* __restrict__ du,
-                               const double* __restrict__ scale) {
+__global__ void k_state_update(DevMesh m, double* U, const double* du,
+                               const double* scale) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
     const int64_t n = m.n;
@@ -325,7 +334,8 @@ __global__ void k_state_update(DevMesh m, double* __restrict__ U, const double* 
     }
 }
 
-__global__ void k_fill(double* __restrict__ x, int64_t count, double value) {
+__global__ void k_fill(double* x, int64_t count, double value) {
+    pdl_enter();
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) x[i] = value;
 }
@@ -334,15 +344,15 @@ __global__ void k_fill(double* __restrict__ x, int64_t count, double value) {
 
 void launch_primitives(const DevMesh& m, const DevFields& f, const GasParams& g, cudaStream_t s) {
     const int64_t th = int64_t(m.n) + m.nb;
-    k_primitives<<<grid_for(th, 256), 256, 0, s>>>(m, f, g);
+    launch_after(k_primitives, grid_for(th, 256), 256, 0, s, m, f, g);
 }
 
 void launch_gradient(const DevMesh& m, const double* src, double* dst, int nvars, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, 128);
     switch (nvars) {
-        case 1: k_gradient<1><<<gr, 128, 0, s>>>(m, src, dst); break;
-        case 5: k_gradient<5><<<gr, 128, 0, s>>>(m, src, dst); break;
-        case 6: k_gradient<6><<<gr, 128, 0, s>>>(m, src, dst); break;  // 5 primitives + nu_tilde
+        case 1: launch_after(k_gradient<1>, gr, 128, 0, s, m, src, dst); break;
+        case 5: launch_after(k_gradient<5>, gr, 128, 0, s, m, src, dst); break;
+        case 6: launch_after(k_gradient<6>, gr, 128, 0, s, m, src, dst); break;  // 5 primitives + nu_tilde
         default: break;
     }
 }
@@ -353,50 +363,51 @@ void launch_limiter_ghostgrad(const DevMesh& m, const DevFields& f, const GasPar
     const int64_t th = int64_t(m.n) + m.nb;
     const unsigned gr = grid_for(th, 128);
     if (!limit) {
-        if (m.nb > 0) k_limiter_ghostgrad<false, 1><<<grid_for(m.nb, 128), 128, 0, s>>>(m, f, g, k3);
+        if (m.nb > 0) launch_after(k_limiter_ghostgrad<false, 1>, grid_for(m.nb, 128), 128, 0, s, m, f, g, k3);
     } else if (limiter == 2) {
-        k_limiter_ghostgrad<true, 2><<<gr, 128, 0, s>>>(m, f, g, k3);
+        launch_after(k_limiter_ghostgrad<true, 2>, gr, 128, 0, s, m, f, g, k3);
     } else if (limiter == 3) {
-        k_limiter_ghostgrad<true, 3><<<gr, 128, 0, s>>>(m, f, g, k3);
+        launch_after(k_limiter_ghostgrad<true, 3>, gr, 128, 0, s, m, f, g, k3);
     } else {
-        k_limiter_ghostgrad<true, 1><<<gr, 128, 0, s>>>(m, f, g, k3);
+        launch_after(k_limiter_ghostgrad<true, 1>, gr, 128, 0, s, m, f, g, k3);
     }
 }
 
 void launch_face_flux(const DevMesh& m, const DevFields& f, const GasParams& g, bool muscl, bool visc,
                       cudaStream_t s) {
     const unsigned gr = grid_for(m.nf, 128);
-    if (muscl && visc) k_face_flux<true, true><<<gr, 128, 0, s>>>(m, f, g);
-    else if (muscl) k_face_flux<true, false><<<gr, 128, 0, s>>>(m, f, g);
-    else if (visc) k_face_flux<false, true><<<gr, 128, 0, s>>>(m, f, g);
-    else k_face_flux<false, false><<<gr, 128, 0, s>>>(m, f, g);
+    if (muscl && visc) launch_after(k_face_flux<true, true>, gr, 128, 0, s, m, f, g);
+    else if (muscl) launch_after(k_face_flux<true, false>, gr, 128, 0, s, m, f, g);
+    else if (visc) launch_after(k_face_flux<false, true>, gr, 128, 0, s, m, f, g);
+    else launch_after(k_face_flux<false, false>, gr, 128, 0, s, m, f, g);
 }
 
 void launch_cell_residual(const DevMesh& m, const DevFields& f, cudaStream_t s) {
-    k_cell_residual<<<grid_for(m.n, 256), 256, 0, s>>>(m, f);
+    launch_after(k_cell_residual, grid_for(m.n, 256), 256, 0, s, m, f);
 }
 
 int norm_blocks(int32_t n) { return static_cast<int>(grid_for(n, 256)); }
 
 void launch_norms(int32_t n, int nv, const double* res, double* partials, double* l2, cudaStream_t s) {
     const unsigned gr = grid_for(n, 256);
-    if (nv == 6) k_norm_partials<6><<<gr, 256, 0, s>>>(n, res, partials);
-    else k_norm_partials<5><<<gr, 256, 0, s>>>(n, res, partials);
-    k_norm_finalize<<<1, 32 * 6, 0, s>>>(static_cast<int>(gr), nv, partials, 1.0 / double(n > 0 ? n : 1), l2);
+    if (nv == 6) launch_after(k_norm_partials<6>, gr, 256, 0, s, n, res, partials);
+    else launch_after(k_norm_partials<5>, gr, 256, 0, s, n, res, partials);
+    launch_after(k_norm_finalize, 1, 32 * 6, 0, s, static_cast<int>(gr), nv, partials, 1.0 / double(n > 0 ? n : 1), l2);
 }
 
 void launch_dt_rhs(const DevMesh& m, const DevFields& f, int nv, double cfl, double diag, double* b, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, 256);
-    if (nv == 6) k_dt_rhs<6><<<gr, 256, 0, s>>>(m, f, cfl, diag, b);
-    else k_dt_rhs<5><<<gr, 256, 0, s>>>(m, f, cfl, diag, b);
+    if (nv == 6) launch_after(k_dt_rhs<6>, gr, 256, 0, s, m, f, cfl, diag, b);
+    else launch_after(k_dt_rhs<5>, gr, 256, 0, s, m, f, cfl, diag, b);
 }
 
 // Dual-time pseudo-source (Solver::add_unsteady_source_term,
 // solver.hpp:546-580): res += V (c0 U + c1 U^n + c2 U^{n-1}); BDF1 has c2 = 0
 // and reads no U^{n-1}.
-__global__ void k_unsteady_source(int32_t n, int nv, const double* __restrict__ vol, const double* __restrict__ U,
-                                  const double* __restrict__ Un, const double* __restrict__ Unm1, double c0,
-                                  double c1, double c2, double* __restrict__ res) {
+__global__ void k_unsteady_source(int32_t n, int nv, const double* vol, const double* U,
+                                  const double* Un, const double* Unm1, double c0,
+                                  double c1, double c2, double* res) {
+    pdl_enter();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (t >= int64_t(n) * nv) return;
     const int32_t c = static_cast<int32_t>(t % n);
@@ -407,18 +418,19 @@ __global__ void k_unsteady_source(int32_t n, int nv, const double* __restrict__ 
 void launch_unsteady_source(int32_t n, int nv, const double* vol, const double* U, const double* Un,
                             const double* Unm1, double c0, double c1, double c2, double* res, cudaStream_t s) {
     const int64_t len = int64_t(n) * nv;
-    if (len > 0) k_unsteady_source<<<grid_for(len, 256), 256, 0, s>>>(n, nv, vol, U, Un, Unm1, c0, c1, c2, res);
+    if (len > 0)
+        launch_after(k_unsteady_source, grid_for(len, 256), 256, 0, s, n, nv, vol, U, Un, Unm1, c0, c1, c2, res);
 }
 
 void launch_state_update(const DevMesh& m, double* U, const double* du, int nv, const double* scale, cudaStream_t s) {
     const unsigned gr = grid_for(m.n, 256);
-    if (nv == 6) k_state_update<6><<<gr, 256, 0, s>>>(m, U, du, scale);
-    else k_state_update<5><<<gr, 256, 0, s>>>(m, U, du, scale);
+    if (nv == 6) launch_after(k_state_update<6>, gr, 256, 0, s, m, U, du, scale);
+    else launch_after(k_state_update<5>, gr, 256, 0, s, m, U, du, scale);
 }
 
 void launch_fill(double* x, int64_t count, double value, cudaStream_t s) {
     if (count <= 0) return;
-    k_fill<<<grid_for(count, 256), 256, 0, s>>>(x, count, value);
+    launch_after(k_fill, grid_for(count, 256), 256, 0, s, x, count, value);
 }
 
 }  // namespace cfdg

@@ -23,7 +23,8 @@ constexpr double kMinWallDist = 1.0e-10;
 // Ghost rho*nu_tilde (SpalartAllmaras::apply_bcs, spalart_allmaras.hpp:234-257)
 // and the pre-sweep (:263-282): density, nu_tilde, eddy viscosity on cells,
 // zero eddy viscosity on BC ghosts.  Threads [0,n) cells, [n,n+nb) ghosts.
-__global__ void k_sa_pre(DevMesh m, DevFields f, GasParams g, SaParams sa, double* __restrict__ rhonu_g) {
+__global__ void k_sa_pre(DevMesh m, DevFields f, GasParams g, SaParams sa, double* rhonu_g) {
+    pdl_enter();
     const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t n = m.n, nt = m.nt;
     if (t < n) {
@@ -58,8 +59,9 @@ __global__ void k_sa_pre(DevMesh m, DevFields f, GasParams g, SaParams sa, doubl
 // faces: owner incl. the ghost's dependence).  A cell's gather then reads
 // one 16-byte pair per face.
 __global__ void __launch_bounds__(128) k_sa_face(DevMesh m, DevFields f, GasParams g, SaParams sa,
-                                                 const double* __restrict__ rhonu_g, const double* __restrict__ gnu,
-                                                 double* __restrict__ out, double* __restrict__ jac) {
+                                                 const double* rhonu_g, const double* gnu,
+                                                 double* out, double* jac) {
+    pdl_enter();
     const int32_t fc = blockIdx.x * blockDim.x + threadIdx.x;
     if (fc >= m.nf) return;
     const int64_t nt = m.nt, nf = m.nf;
@@ -130,8 +132,9 @@ __global__ void __launch_bounds__(128) k_sa_face(DevMesh m, DevFields f, GasPara
 // sequential reference), spectral radius increments, and the cell sources
 // (SpalartAllmaras::cell_sources, spalart_allmaras.hpp:376-432); dsrc = the
 // destruction derivative V 2 cw1 fw nu / d^2 for the Jacobian diagonal.
-__global__ void __launch_bounds__(128) k_sa_cell(DevMesh m, DevFields f, SaParams sa, const double* __restrict__ face,
-                                                 const double* __restrict__ gnu, double* __restrict__ dsrc) {
+__global__ void __launch_bounds__(128) k_sa_cell(DevMesh m, DevFields f, SaParams sa, const double* face,
+                                                 const double* gnu, double* dsrc) {
+    pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n) return;
     const int64_t nt = m.nt, n = m.n;
@@ -139,7 +142,7 @@ __global__ void __launch_bounds__(128) k_sa_cell(DevMesh m, DevFields f, SaParam
     for (int32_t e = m.c2f_off[c]; e < m.c2f_off[c + 1]; ++e) {
         const int32_t es = __ldg(m.c2fs + e);  // the side is in the sign: no owner gather
         const int32_t fc = es >= 0 ? es : ~es;
-        const double2 fr = __ldg(reinterpret_cast<const double2*>(face) + fc);
+        const double2 fr = reinterpret_cast<const double2*>(face)[fc];
         if (es >= 0) r += fr.x;
         else r -= fr.x;
         if (fc < m.ni) l += fr.y;
@@ -179,14 +182,14 @@ __global__ void __launch_bounds__(128) k_sa_cell(DevMesh m, DevFields f, SaParam
 
 void launch_sa_pre(const DevMesh& m, const DevFields& f, const GasParams& g, const SaParams& sa, double* rhonu_g,
                    cudaStream_t s) {
-    k_sa_pre<<<grid_for(int64_t(m.n) + m.nb, 256), 256, 0, s>>>(m, f, g, sa, rhonu_g);
+    launch_after(k_sa_pre, grid_for(int64_t(m.n) + m.nb, 256), 256, 0, s, m, f, g, sa, rhonu_g);
 }
 
 void launch_sa_sweep(const DevMesh& m, const DevFields& f, const GasParams& g, const SaParams& sa,
                      const double* rhonu_g, const double* gnu, double* face, double* jac, double* dsrc,
                      cudaStream_t s) {
-    k_sa_face<<<grid_for(m.nf, 128), 128, 0, s>>>(m, f, g, sa, rhonu_g, gnu, face, jac);
-    k_sa_cell<<<grid_for(m.n, 128), 128, 0, s>>>(m, f, sa, face, gnu, dsrc);
+    launch_after(k_sa_face, grid_for(m.nf, 128), 128, 0, s, m, f, g, sa, rhonu_g, gnu, face, jac);
+    launch_after(k_sa_cell, grid_for(m.n, 128), 128, 0, s, m, f, sa, face, gnu, dsrc);
 }
 
 

@@ -17,6 +17,7 @@
 
 #include <algorithm>
 
+#include "device_common.cuh"
 #include "mlp.hpp"
 #include "tcgen05.cuh"
 
@@ -29,7 +30,7 @@ constexpr uint32_t kWaitLimit = 1u << 26;  // mbarrier polls before a wait gives
 __device__ __forceinline__ uint16_t f2bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 
 // Row-major bf16 [R x K] (global) -> K-major core tile; rows >= valid are zero.
-__device__ void load_tile(uint8_t* tile, const uint16_t* __restrict__ g, int R, int K, int64_t valid) {
+__device__ void load_tile(uint8_t* tile, const uint16_t* g, int R, int K, int64_t valid) {
     const int kc = K >> 3;
     for (int q = threadIdx.x; q < R * kc; q += blockDim.x) {
         const int r = q / kc, c = q - r * kc;
@@ -229,9 +230,10 @@ __device__ __forceinline__ uint64_t epi_hidden_t(uint32_t tacc, const float* bia
 }
 
 // ----------------------------------------------------------- inference
-__global__ void __launch_bounds__(128) k_mlp_forward(MlpDev net, const uint16_t* __restrict__ feat, int64_t rows,
-                                                     const double* __restrict__ scale, int nv,
-                                                     double* __restrict__ out, int* err) {
+__global__ void __launch_bounds__(128) k_mlp_forward(MlpDev net, const uint16_t* feat, int64_t rows,
+                                                     const double* scale, int nv,
+                                                     double* out, int* err) {
+    pdl_enter();
     extern __shared__ __align__(128) uint8_t smem[];
     const FwdSmem s = carve_fwd(smem);
     load_net(net, s.w1, s.w2, s.w3, s.bias);
@@ -338,9 +340,10 @@ __device__ TrainSmem carve_train(uint8_t* smem) {
 // written from registers, and the partials leave as 16-byte words.  With the
 // losses read once an epoch, one epoch of 8,192-sample batches over 600,011
 // samples went from 5.0 to 1.75 ms (68 to 24 us a batch).
-__global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t* __restrict__ feat,
-                                                     const float* __restrict__ target, int64_t rows,
-                                                     float* __restrict__ partials, int* err) {
+__global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t* feat,
+                                                     const float* target, int64_t rows,
+                                                     float* partials, int* err) {
+    pdl_enter();
     extern __shared__ __align__(128) uint8_t smem[];
     const TrainSmem s = carve_train(smem);
     if (__syncthreads_or(*err != 0)) return;  // an earlier batch failed: the host reports it
@@ -382,10 +385,10 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
         float tv[kMlpOut];
 #pragma unroll
         for (int c = 0; c < kMlpIn / 8; ++c)
-            xv[c] = valid ? __ldg(reinterpret_cast<const uint4*>(feat + (r0 + r) * kMlpIn) + c) : make_uint4(0u, 0u, 0u, 0u);
+            xv[c] = valid ? reinterpret_cast<const uint4*>(feat + (r0 + r) * kMlpIn)[c] : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
         for (int c = 0; c < kMlpOut / 4; ++c) {
-            const float4 q = valid ? __ldg(reinterpret_cast<const float4*>(target + (r0 + r) * kMlpOut) + c)
+            const float4 q = valid ? reinterpret_cast<const float4*>(target + (r0 + r) * kMlpOut)[c]
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
             tv[4 * c] = q.x;
             tv[4 * c + 1] = q.y;
@@ -539,16 +542,17 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
 constexpr int kAdamParams = 32, kAdamSlices = 8;
 
 __global__ void __launch_bounds__(kAdamParams * kAdamSlices)
-    k_mlp_adam(float* params, float* m, float* v, uint16_t* __restrict__ w, const float* __restrict__ partials,
+    k_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials,
                int nparts, double inv_count, float lr, float b1, float b2, float eps, float c1, float c2, bool adam,
                float* grad_out, float* loss_out) {
+    pdl_enter();
     __shared__ double sh[kAdamSlices][kAdamParams];
     const int local = threadIdx.x % kAdamParams, slice = threadIdx.x / kAdamParams;
     const int p = blockIdx.x * kAdamParams + local;
     double part = 0.0;
     if (p <= kMlpParams) {
 #pragma unroll 8
-        for (int c = slice; c < nparts; c += kAdamSlices) part += double(__ldg(partials + int64_t(c) * kMlpPartials + p));
+        for (int c = slice; c < nparts; c += kAdamSlices) part += double(partials[int64_t(c) * kMlpPartials + p]);
     }
     sh[slice][local] = part;
     __syncthreads();
@@ -597,7 +601,7 @@ void launch_mlp_forward(const MlpDev& net, const uint16_t* feat, int64_t rows, c
     cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
     const int64_t ntiles = (rows + kMlpTile - 1) / kMlpTile;
     const int g = static_cast<int>(std::min<int64_t>(ntiles, grid));
-    k_mlp_forward<<<g, 128, kFwdSmem, s>>>(net, feat, rows, scale, nv, out, err);
+    launch_after(k_mlp_forward, g, 128, kFwdSmem, s, net, feat, rows, scale, nv, out, err);
 }
 
 int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target, int64_t rows, float* partials,
@@ -605,7 +609,7 @@ int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target
     cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrainSmem);
     const int64_t ntiles = (rows + kMlpTile - 1) / kMlpTile;
     const int g = static_cast<int>(std::min<int64_t>(ntiles, grid));
-    k_mlp_grad<<<g, 128, kTrainSmem, s>>>(net, feat, target, rows, partials, err);
+    launch_after(k_mlp_grad, g, 128, kTrainSmem, s, net, feat, target, rows, partials, err);
     return g;
 }
 
@@ -613,8 +617,8 @@ void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float
                      double inv_count, float lr, float beta1, float beta2, float eps, int step, bool adam,
                      float* grad_out, float* loss_out, cudaStream_t s) {
     const float c1 = 1.0f - powf(beta1, float(step)), c2 = 1.0f - powf(beta2, float(step));
-    k_mlp_adam<<<(kMlpParams + kAdamParams) / kAdamParams, kAdamParams * kAdamSlices, 0, s>>>(
-        params, m, v, w, partials, nparts, inv_count, lr, beta1, beta2, eps, c1, c2, adam, grad_out, loss_out);
+    launch_after(k_mlp_adam, (kMlpParams + kAdamParams) / kAdamParams, kAdamParams * kAdamSlices, 0, s, params, m, v, w,
+                 partials, nparts, inv_count, lr, beta1, beta2, eps, c1, c2, adam, grad_out, loss_out);
 }
 
 }  // namespace cfdg
