@@ -631,6 +631,7 @@ int cfdg_mlp_forward_host(cfdg_mlp* m, const uint16_t* feat_h, int64_t rows, dou
             const double ones[8] = {1, 1, 1, 1, 1, 1, 1, 1};
             cfdg::cuda_check(cudaMemcpy(S, ones, sizeof(ones), cudaMemcpyHostToDevice), "H2D");
             cfdg::cuda_check(cudaMemcpy(F, feat_h, rows * cfdg::kMlpIn * 2, cudaMemcpyHostToDevice), "H2D");
+            cfdg::default_stream_done();
             m->impl->forward(F, rows, S, O, m->stream);
             cfdg::cuda_check(cudaStreamSynchronize(m->stream), "sync");
             cfdg::cuda_check(cudaMemcpy(out_h, O, rows * nv * 8, cudaMemcpyDeviceToHost), "D2H");

@@ -31,6 +31,10 @@ uint16_t to_bf16(float x) {  // round to nearest even (finite inputs)
 
 }  // namespace
 
+// cudaMemcpy from pageable memory returns once the data is staged, and the
+// kernels run on streams that do not wait for the default one.
+void default_stream_done() { cuda_check(cudaStreamSynchronize(nullptr), "H2D sync"); }
+
 Mlp::Mlp(int device, int nvars, uint64_t seed) : device_(device), nvars_(nvars) {
     if (nvars < 1 || nvars > kMlpOut || 8 * nvars > kMlpIn)
         throw Failure{CFDG_ERR_INVALID, "learned guess supports 1..6 variables"};
@@ -101,6 +105,7 @@ void Mlp::set_params(const float* p) {
     step_ = 0;
     cuda_check(cudaMemset(m_, 0, kMlpParams * sizeof(float)), "memset");
     cuda_check(cudaMemset(v_, 0, kMlpParams * sizeof(float)), "memset");
+    default_stream_done();
 }
 
 void Mlp::get_params(float* p) {
@@ -214,6 +219,7 @@ void Dataset::append_host(const uint16_t* X, const float* T, int64_t rows) {
     if (g < rows) throw Failure{CFDG_ERR_INVALID, "dataset capacity exceeded"};
     cuda_check(cudaMemcpy(X_ + r0 * kMlpIn, X, rows * kMlpIn * sizeof(uint16_t), cudaMemcpyHostToDevice), "H2D");
     cuda_check(cudaMemcpy(T_ + r0 * kMlpOut, T, rows * kMlpOut * sizeof(float), cudaMemcpyHostToDevice), "H2D");
+    default_stream_done();
 }
 
 void Dataset::read_host(uint16_t* X, float* T, int64_t rows) const {

@@ -24,6 +24,8 @@ void launch_guess_append(int32_t n, const int32_t* row_of, int nv, int32_t strid
 
 class Dataset;
 
+void default_stream_done();  // what was copied on the default stream has arrived
+
 class Mlp {
 public:
     Mlp(int device, int nvars, uint64_t seed);
