@@ -52,9 +52,10 @@ __global__ void k_primitives(DevMesh m, DevFields f, GasParams g) {
 // the latency of the gathers; with seven blocks an SM (72 registers; the
 // compiler took 80) five variables of a 131k-cell hex mesh, 27 cells a stencil,
 // take 34 us instead of 52, of 1M cells 226 instead of 248, of 768k
-// tetrahedra 390 instead of 435; eight or more blocks spill.
+// tetrahedra 390 instead of 435; eight or more blocks spill, and so do six
+// variables at seven (0.92 -> 1.17 ms on 4.1M cells), which keep the compiler's.
 template <int NVG>
-__global__ void __launch_bounds__(128, 7) k_gradient(DevMesh m, const double* src, double* dst) {
+__global__ void __launch_bounds__(128, NVG <= 5 ? 7 : 0) k_gradient(DevMesh m, const double* src, double* dst) {
     pdl_enter();
     const int32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const int32_t slice = c >> 5;
