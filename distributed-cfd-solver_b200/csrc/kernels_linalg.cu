@@ -715,6 +715,45 @@ __global__ void __launch_bounds__(256, BS <= 5 ? 6 : 5) k_sgs_last_spmv(BsrView 
     if constexpr (ND > 0) block_reduce_store<ND, 256>(pr, partials + size_t(blockIdx.x) * ND);
 }
 
+// The inner products that k_sgs_last_spmv (the first g0 blocks: colour 0 as
+// warps of 32 / BS rows) and k_spmv (the others: the components after it) form
+// with their results: the same blocks, the same order, the same partials to the
+// bit.  Bound by the vectors' traffic.
+template <int BS, int ND>
+__global__ void __launch_bounds__(kVecThreads) k_dots(int32_t n0, int32_t n, int g0, const double* __restrict__ y,
+                                                      DotSpec ds, double* __restrict__ partials,
+                                                      const int* __restrict__ active) {
+    if (active && *active != 0) return;
+    double pr[ND];
+#pragma unroll
+    for (int k = 0; k < ND; ++k) pr[k] = 0.0;
+    auto add = [&](int64_t t) {
+        const double yv = y[t];
+#pragma unroll
+        for (int k = 0; k < ND; ++k) {
+            const double a = ds.a[k] ? ds.a[k][t] : yv;
+            const double b = ds.b[k] ? ds.b[k][t] : yv;
+            pr[k] += a * b;
+        }
+    };
+    if (static_cast<int>(blockIdx.x) < g0) {
+        constexpr int GPW = 32 / BS;
+        const int lane = threadIdx.x & 31, grp = lane / BS, ii = lane - grp * BS;
+        const int64_t warps = (int64_t(g0) * kVecThreads) >> 5;
+#pragma unroll 4
+        for (int64_t w = (int64_t(blockIdx.x) * kVecThreads + threadIdx.x) >> 5; w * GPW < n0; w += warps) {
+            const int64_t row = w * GPW + grp;
+            if (grp < GPW && row < n0) add(row * BS + ii);
+        }
+    } else {
+        const int64_t stride = int64_t(gridDim.x - g0) * kVecThreads, N = int64_t(n) * BS;
+#pragma unroll 4
+        for (int64_t t = int64_t(n0) * BS + int64_t(blockIdx.x - g0) * kVecThreads + threadIdx.x; t < N; t += stride)
+            add(t);
+    }
+    block_reduce_store<ND, kVecThreads>(pr, partials + size_t(blockIdx.x) * ND);
+}
+
 // ------------------------------------------------------ Krylov kernels
 // r = b - v (v null: r = b), r0 = r, p = r; partial sums of |b|^2 and |r|^2.
 __global__ void __launch_bounds__(kVecThreads) k_krylov_init(int64_t len, const double* __restrict__ b,
@@ -1149,6 +1188,21 @@ template bool launch_sgs_level_cluster<double>(const BsrView&, const double*, co
 template bool launch_sgs_level_cluster<float>(const BsrView&, const float*, const float*, const int8_t*, const int4*,
                                               const int32_t*, int, const int4*, const int32_t*, int, const double*,
                                               double*, bool, int, int, const int*, cudaStream_t);
+
+int launch_dots(int32_t n0, int32_t n, int bs, const double* y, const DotSpec& ds, double* partials, const int* active,
+                cudaStream_t s) {
+    const int g0 = n0 > 0 ? sgs_last_spmv_blocks(n0, bs) : 0, g = g0 + spmv_blocks(n - n0, bs);
+    auto go = [&](auto bsc, auto nd) {
+        k_dots<decltype(bsc)::value, decltype(nd)::value><<<g, kVecThreads, 0, s>>>(n0, n, g0, y, ds, partials, active);
+    };
+    auto by_nd = [&](auto bsc) {
+        if (ds.n == 1) go(bsc, std::integral_constant<int, 1>{});
+        else go(bsc, std::integral_constant<int, 5>{});
+    };
+    if (bs == 6) by_nd(std::integral_constant<int, 6>{});
+    else by_nd(std::integral_constant<int, 5>{});
+    return g;
+}
 
 int dot_blocks(int64_t len) { return static_cast<int>(vec_grid(len)); }
 

@@ -112,6 +112,34 @@ bool launch_sgs_level_cluster(const BsrView& A, const MT* vals, const MT* lu, co
                               const int32_t* fwd_off, int n_fwd, const int4* bwd_rows, const int32_t* bwd_off,
                               int n_bwd, const double* r, double* z, bool from_zero, int C, int smem,
                               const int* active, cudaStream_t s);
+// A colour-ordered system in slices of 32 rows (kernels_sell.cu).  Slot
+// (slice, lane) holds row[slot] (-1: none) with len[slot] blocks below and above
+// the diagonal; column c of the values is 32 blocks, entry e of lane l at
+// (c * bs^2 + e) * 32 + l, cols[c * 32 + l] the block's column.  desc[slice]:
+// first lower column, their count, first upper column, their count; its diagonal
+// blocks are column diag0 + slice, its D^-1 column `slice` of their array.
+struct SellView {
+    int32_t bs, diag0;
+    const int32_t *row, *cols;
+    const int2* len;
+    const int4* desc;
+};
+// Passes (z the vector the neighbour blocks multiply):
+//   DIAG  z = D^-1 r            LOW  z = D^-1 (r - L z)   FULL  z = D^-1 (r - L z - U z)
+//   UP    z += D^-1 (-U z)      UPY  as UP, and y = U z + D z (the row's product when L is empty)
+//   MUL   y = A z
+enum : int { SELL_DIAG, SELL_LOW, SELL_UP, SELL_UPY, SELL_FULL, SELL_MUL };
+// Whether the device can run the passes (asked once, outside a capture).
+bool sell_ready(int bs, bool mixed);
+template <typename MT>
+void launch_sell_copy(int bs, int64_t columns, const int32_t* src, const MT* from, MT* to, cudaStream_t s);
+template <typename MT>
+void launch_sell_rows(const SellView& A, const MT* vals, const MT* dinv, int kind, int32_t s0, int32_t s1,
+                      const double* r, double* z, double* y, const int* active, cudaStream_t s);
+// Inner products of y = A z as k_sgs_last_spmv (rows [0, n0), n0 = 0: none) and
+// k_spmv (the rest) sum them; returns the partial rows.
+int launch_dots(int32_t n0, int32_t n, int bs, const double* y, const DotSpec& ds, double* partials, const int* active,
+                cudaStream_t s);
 void launch_krylov_init(int64_t len, const double* b, const double* v, double* r, double* r0, double* p,
                         double* partials, KrylovScalars* ks, cudaStream_t s);
 // After launch_krylov_init: a rejected initial guess (||b - A x0|| >=

@@ -339,7 +339,8 @@ __device__ TrainSmem carve_train(uint8_t* smem) {
 // in as 16-byte words in both orientations, the transposed operands are
 // written from registers, and the partials leave as 16-byte words.  With the
 // losses read once an epoch, one epoch of 8,192-sample batches over 600,011
-// samples went from 5.0 to 1.75 ms (68 to 24 us a batch).
+// samples went from 5.0 to 1.75 ms, with dependent launches to 1.56 (68 to 21 us
+// a batch).
 __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t* feat,
                                                      const float* target, int64_t rows,
                                                      float* partials, int* err) {

@@ -280,6 +280,7 @@ void BsrSystem::set_precision(int precision) {
     if (precision == precision_) return;
     const std::size_t nv = static_cast<std::size_t>(nnzb_) * bs_ * bs_;
     release_device_loop();  // the captured iterations launch precision-specific kernels
+    release_sell();
     release_red_graphs();
     if (precision == CFDG_PREC_MIXED) {
         vals64_.release();
@@ -618,6 +619,9 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
         launch_lu_setup<double>(view(), vals64_.p, lu64_.p, nullptr, piv_.p, err_.p, color, stream_);
     }
     cuda_check(cudaGetLastError(), "lu launch");
+    const bool was = sell_on_;
+    fill_sell();
+    if (was != sell_on_) release_device_loop();  // the captured iteration's passes change
     lu_ready_ = true;
     lu_unchecked_ = true;
     if (check) {
@@ -642,6 +646,143 @@ void BsrSystem::check_factorisation() {
     if (err > 0)
         throw Failure{CFDG_ERR_SINGULAR, "SgsPreconditioner: singular diagonal block at row " + std::to_string(err - 1)};
     throw Failure{CFDG_ERR_NONFINITE, "SgsPreconditioner: non-finite diagonal block at row " + std::to_string(-err - 1)};
+}
+
+// Where the sliced copy pays: the copy costs a read and a write of the matrix
+// per set-up, and its passes need many slices.  At twice L2 it is ahead (370 MB
+// of 6x6 FP32 blocks: 18.0 -> 15.9 ms a step), at 178 MB (131k hex cells, FP64,
+// four iterations a solve) 2% behind, at 48 MB 25%.  Row by row, FP32 blocks of
+// both sizes and FP64 5x5 ones are bound by L1 wavefronts; FP64 6x6 ones run at
+// 0.94 of the copy bandwidth and stay.
+constexpr double kSellMin = 2 * 126e6;
+bool BsrSystem::sell_wanted() const {
+    return sliced && !sell_failed_ && ordering_ == CFDG_SGS_COLOR && split_ && groups_bwd() >= 2 &&
+           (bs_ == 5 || (bs_ == 6 && precision_ == CFDG_PREC_MIXED)) && double(nnzb_) * block_bytes() > kSellMin &&
+           !reducible();
+}
+
+// Slices of the ordering.
+void BsrSystem::build_sell() {
+    const int ng = groups_fwd();
+    std::vector<int32_t> row;
+    row.reserve(static_cast<std::size_t>(n_) + 32 * ng);
+    sell_first_.assign(1, 0);
+    for (int g = 0; g < ng; ++g) {
+        for (int32_t a = fwd_off_[g]; a < fwd_off_[g + 1]; a += 256) {
+            const int32_t b = std::min(a + 256, fwd_off_[g + 1]);
+            const std::size_t at = row.size();
+            for (int32_t i = a; i < b; ++i) row.push_back(i);
+            auto key = [&](int32_t i) {  // blocks below, then above
+                return int64_t(diag_h_[i] - row_ptr_h_[i]) << 32 | int64_t(row_ptr_h_[i + 1] - diag_h_[i]);
+            };
+            std::stable_sort(row.begin() + at, row.end(), [&](int32_t p, int32_t q) { return key(p) > key(q); });
+        }
+        while (row.size() % 32) row.push_back(-1);
+        sell_first_.push_back(static_cast<int32_t>(row.size() / 32));
+    }
+    const std::size_t ns = row.size() / 32;
+    std::vector<int2> len(row.size(), make_int2(0, 0));
+    std::vector<int4> desc(ns, make_int4(0, 0, 0, 0));
+    int32_t c = 0;
+    for (std::size_t s = 0; s < ns; ++s) {
+        int4& d = desc[s];
+        for (std::size_t q = s * 32; q < s * 32 + 32; ++q) {
+            const int32_t i = row[q];
+            if (i < 0) continue;
+            len[q] = make_int2(diag_h_[i] - row_ptr_h_[i], row_ptr_h_[i + 1] - diag_h_[i] - 1);
+            d.y = std::max(d.y, len[q].x);
+            d.w = std::max(d.w, len[q].y);
+        }
+        d.x = c;
+        d.z = c + d.y;
+        c += d.y + d.w;
+    }
+    sell_diag0_ = c;
+    sell_columns_ = c + static_cast<int64_t>(ns);
+    std::vector<int32_t> src(static_cast<std::size_t>(sell_columns_) * 32, -1), cols(src.size(), 0);
+    for (std::size_t s = 0; s < ns; ++s) {
+        const int4 d = desc[s];
+        for (int l = 0; l < 32; ++l) {
+            const int32_t i = row[s * 32 + l];
+            if (i < 0) continue;
+            for (int32_t k = row_ptr_h_[i]; k < row_ptr_h_[i + 1]; ++k) {
+                const int64_t at = k < diag_h_[i]    ? d.x + (k - row_ptr_h_[i])
+                                   : k == diag_h_[i] ? sell_diag0_ + static_cast<int64_t>(s)
+                                                     : d.z + (k - diag_h_[i] - 1);
+                src[at * 32 + l] = k;
+                cols[at * 32 + l] = cols_h_[k];
+            }
+        }
+    }
+    upload_or_throw(sell_row_, row, stream_, "slices");
+    upload_or_throw(sell_cols_, cols, stream_, "slices");
+    upload_or_throw(sell_src_, src, stream_, "slices");
+    upload_or_throw(sell_len_, len, stream_, "slices");
+    upload_or_throw(sell_desc_, desc, stream_, "slices");
+    cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // the host arrays die here
+    sell_ordering_ = ordering_;
+}
+
+// The sliced copy of the current values and diagonal inverses.
+void BsrSystem::fill_sell() {
+    sell_on_ = false;
+    if (!sell_wanted()) return;
+    const int64_t b2 = int64_t(bs_) * bs_;
+    try {
+        if (!sell32_.p && !sell64_.p) {  // a second copy of the matrix only where memory is ample
+            std::size_t room = 0, total = 0;
+            cuda_check(cudaMemGetInfo(&room, &total), "cudaMemGetInfo");
+            if (!sell_ready(bs_, precision_ == CFDG_PREC_MIXED) || 8.0 * double(nnzb_) * block_bytes() > double(room)) {
+                sell_failed_ = true;
+                return;
+            }
+        }
+        if (sell_ordering_ != ordering_) build_sell();
+        const std::size_t nv = static_cast<std::size_t>(sell_columns_ * 32 * b2),
+                          ni = static_cast<std::size_t>((sell_columns_ - sell_diag0_) * 32 * b2);
+        if (precision_ == CFDG_PREC_MIXED) {
+            if (!sell32_.p) alloc_or_throw(sell32_, nv, "slices");
+            if (!sellinv32_.p) alloc_or_throw(sellinv32_, ni, "slices");
+        } else {
+            if (!sell64_.p) alloc_or_throw(sell64_, nv, "slices");
+            if (!sellinv64_.p) alloc_or_throw(sellinv64_, ni, "slices");
+        }
+    } catch (const Failure& f) {
+        if (f.status != CFDG_ERR_NOMEM) throw;
+        cudaGetLastError();  // no room for a second copy: the passes read the matrix itself
+        release_sell();
+        sell_failed_ = true;
+        return;
+    }
+    ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 2, 2.0 * (double(nnzb_) + n_) * block_bytes());
+    // a diagonal column's sources are blocks; its rows index the inverses
+    if (precision_ == CFDG_PREC_MIXED) {
+        launch_sell_copy<float>(bs_, sell_columns_, sell_src_.p, vals32_.p, sell32_.p, stream_);
+        launch_sell_copy<float>(bs_, sell_columns_ - sell_diag0_, sell_row_.p, lu32_.p, sellinv32_.p, stream_);
+    } else {
+        launch_sell_copy<double>(bs_, sell_columns_, sell_src_.p, vals64_.p, sell64_.p, stream_);
+        launch_sell_copy<double>(bs_, sell_columns_ - sell_diag0_, sell_row_.p, lu64_.p, sellinv64_.p, stream_);
+    }
+    cuda_check(cudaGetLastError(), "slice copy launch");
+    sell_on_ = true;
+}
+
+void BsrSystem::release_sell() {
+    sell_on_ = false;
+    sell64_.release();
+    sellinv64_.release();
+    sell32_.release();
+    sellinv32_.release();
+}
+
+// A pass over the colours [c0, c1).
+void BsrSystem::sell_pass(int kind, int c0, int c1, const double* r, double* z, double* y, const int* active) {
+    const SellView A{bs_, static_cast<int32_t>(sell_diag0_), sell_row_.p, sell_cols_.p, sell_len_.p, sell_desc_.p};
+    const int32_t s0 = sell_first_[c0], s1 = sell_first_[c1];
+    if (precision_ == CFDG_PREC_MIXED)
+        launch_sell_rows<float>(A, sell32_.p, sellinv32_.p, kind, s0, s1, r, z, y, active, stream_);
+    else
+        launch_sell_rows<double>(A, sell64_.p, sellinv64_.p, kind, s0, s1, r, z, y, active, stream_);
 }
 
 template <typename MT>
@@ -688,6 +829,11 @@ void BsrSystem::sgs_apply_t(const MT* vals, const MT* lu, const double* r, doubl
                 if (sw == 0) mode = (g == 0) ? 1 : (split ? 2 : 0);  // colour 0: all neighbours still zero
             }
             ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, fwd_bytes_[mode][g] + fwd_blocks_[mode][g] * block_bytes());
+            if (sell_on_) {
+                static constexpr int kinds[3] = {SELL_FULL, SELL_DIAG, SELL_LOW};
+                sell_pass(kinds[mode], g, g + 1, r, z, nullptr, active);
+                continue;
+            }
             const bool cg = fwd_first_[g] >= 0;
             launch_sgs_rows_ex<MT>(A, vals, lu, piv_.p, cg ? nullptr : fwd_rows_.p + fwd_off_[g], cg ? fwd_first_[g] : 0,
                                    fwd_off_[g + 1] - fwd_off_[g], r, z, mode, color, active, stream_);
@@ -697,6 +843,10 @@ void BsrSystem::sgs_apply_t(const MT* vals, const MT* lu, const double* r, doubl
             if (skip_last && g == nbk - 1) continue;  // fused with the product (sgs_apply_spmv)
             ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1,
                          bwd_bytes_[split ? 2 : 0][g] + bwd_blocks_[split ? 2 : 0][g] * block_bytes());
+            if (sell_on_) {  // backward group g is colour nbk - 1 - g
+                sell_pass(split ? SELL_UP : SELL_FULL, nbk - 1 - g, nbk - g, r, z, nullptr, active);
+                continue;
+            }
             const bool cg = bwd_first_[g] >= 0;
             launch_sgs_rows_ex<MT>(A, vals, lu, piv_.p, cg ? nullptr : bwd_rows_.p + bwd_off_[g], cg ? bwd_first_[g] : 0,
                                    bwd_off_[g + 1] - bwd_off_[g], r, z, split ? 3 : 0, color, active, stream_);
@@ -712,6 +862,29 @@ int BsrSystem::sgs_apply_spmv(const double* r, double* z, double* y, const DotSp
     const double sa = mixed ? 4.0 : 8.0;
     const double b2 = double(bs_) * bs_;
     const int nx = ds.n == 1 ? 1 : 2;  // vectors the dots read besides y (r0; r0 and s)
+    if (sell_on_) {
+        const bool fuse = fuse_last_spmv();
+        const int32_t n0 = fuse ? fwd_off_[1] : 0;
+        if (mixed) sgs_apply_t<float>(vals32_.p, lu32_.p, r, z, active, fuse);
+        else sgs_apply_t<double>(vals64_.p, lu64_.p, r, z, active, fuse);
+        if (fuse) {
+            ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1,
+                         bwd_bytes_[2][groups_bwd() - 1] + bwd_blocks_[2][groups_bwd() - 1] * block_bytes() +
+                             double(n0) * (b2 * sa + bs_ * 8.0));
+            sell_pass(SELL_UPY, 0, 1, nullptr, z, y, active);
+        }
+        {
+            const double Nr = double(n_ - n0) * bs_;
+            ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1,
+                         fuse ? rest_nnzb_ * (b2 * sa + 4.0) + rest_cols_ * bs_ * 8.0 + Nr * 8.0
+                              : spmv_bytes(0, false));
+            sell_pass(SELL_MUL, fuse ? 1 : 0, groups_fwd(), nullptr, z, y, active);
+        }
+        ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, double(n_) * bs_ * 8.0 * (1.0 + nx));
+        const int parts = launch_dots(n0, n_, bs_, y, ds, partials, active, stream_);
+        cuda_check(cudaGetLastError(), "sgs+spmv launch");
+        return parts;
+    }
     if (!fuse_last_spmv()) {
         sgs_apply(r, z, active);
         ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, spmv_bytes(nx, false));
@@ -1732,6 +1905,7 @@ void Solver::setup_matrix(const HostMesh& hm, const Csr& c2c) {
     sys_ = std::make_unique<BsrSystem>(device_, n, nv_, row_ptr.data(), cols.data(),
                                        pre_freeze_phase() ? CFDG_PREC_FP64 : cfg_.precision, stream_);
     sys_->device_loop = cfg_.krylov_loop == CFDG_KRYLOV_DEVICE_LOOP;
+    sys_->sliced = sys_->device_loop;  // the host loop keeps the row-by-row kernels
     // The reduced solve has the iterates of the full one up to rounding.  On
     // the wall-stretched viscous systems an unconverged solve amplifies
     // rounding up to 1e13 times (two solves whose input differs by one unit in

@@ -193,6 +193,7 @@ public:
     bool device_loop = true;  // run the iterations as one graph launch (CFDG_KRYLOV_DEVICE_LOOP)
     // Systems whose multicolour BiCGSTAB runs in its reduced form
     // (kernels_reduced.cu).
+    bool sliced = false;  // keep a sliced copy of the matrix where that pays (the owner refills the values each solve)
     enum Reduce { REDUCE_NONE, REDUCE_FP64, REDUCE_ANY };
     Reduce reduce = REDUCE_ANY;
 
@@ -207,6 +208,21 @@ private:
     void sgs_apply_t(const MT* vals, const MT* lu, const double* r, double* z, const int* active,
                      bool skip_last = false);
     bool fuse_last_spmv() const { return split_ && sweeps_ == 1 && groups_bwd() >= 2; }
+    // Sliced copy of the matrix for the sweeps (kernels_sell.cu).
+    bool sell_wanted() const;
+    void build_sell();
+    void fill_sell();
+    void release_sell();
+    void sell_pass(int kind, int c0, int c1, const double* r, double* z, double* y, const int* active);
+    bool sell_on_ = false, sell_failed_ = false;
+    int sell_ordering_ = -1;
+    std::vector<int32_t> sell_first_;  // first slice of each colour
+    int64_t sell_columns_ = 0, sell_diag0_ = 0;
+    DevArray<int32_t> sell_row_, sell_cols_, sell_src_;
+    DevArray<int2> sell_len_;
+    DevArray<int4> sell_desc_;
+    DevArray<double> sell64_, sellinv64_;
+    DevArray<float> sell32_, sellinv32_;
     // BiCGSTAB + one multicolour sweep on the rows outside the first colour
     // (kernels_reduced.cu)
     bool reducible() const {
