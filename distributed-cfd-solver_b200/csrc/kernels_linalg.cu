@@ -177,17 +177,16 @@ constexpr int kLuThreads = 128;
 // column of a thread spill below ~170 registers, the 5x5 ones below ~128.
 template <typename MT, int BS, bool INV>
 __global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, const MT* vals, MT* lu,
-                                                   double* inv64, int8_t* piv,
-                                                   int* err) {
+                                                   int8_t* piv, int* err) {
     pdl_enter();
     constexpr int B2 = BS * BS;
     constexpr int SP = B2 % 2 == 0 ? B2 + 1 : B2;  // odd row stride: thread-per-row accesses hit distinct banks
-    __shared__ double sm[kLuThreads * SP];
+    __shared__ MT sm[kLuThreads * SP];
     const int32_t r0 = blockIdx.x * kLuThreads;
     const int32_t nrows = min(kLuThreads, A.n - r0);
     for (int q = threadIdx.x; q < nrows * B2; q += kLuThreads) {
         const int row = q / B2, e = q - row * B2;
-        sm[row * SP + e] = static_cast<double>(vals[int64_t(A.diag[r0 + row]) * B2 + e]);
+        sm[row * SP + e] = vals[int64_t(A.diag[r0 + row]) * B2 + e];
     }
     __syncthreads();
     const int32_t i = r0 + threadIdx.x;
@@ -195,7 +194,7 @@ __global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, c
     double a[BS * BS];
     if (act) {
 #pragma unroll
-        for (int e = 0; e < BS * BS; ++e) a[e] = sm[threadIdx.x * SP + e];
+        for (int e = 0; e < BS * BS; ++e) a[e] = static_cast<double>(sm[threadIdx.x * SP + e]);
     } else {
 #pragma unroll
         for (int e = 0; e < BS * BS; ++e) a[e] = (e % (BS + 1) == 0) ? 1.0 : 0.0;
@@ -270,11 +269,11 @@ __global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, c
                     x[r] = x[r] * rd[r];
                 }
 #pragma unroll
-                for (int r = 0; r < BS; ++r) sm[threadIdx.x * SP + r * BS + c] = x[r];
+                for (int r = 0; r < BS; ++r) sm[threadIdx.x * SP + r * BS + c] = static_cast<MT>(x[r]);
             }
         } else {
 #pragma unroll
-            for (int e = 0; e < BS * BS; ++e) sm[threadIdx.x * SP + e] = a[e];
+            for (int e = 0; e < BS * BS; ++e) sm[threadIdx.x * SP + e] = static_cast<MT>(a[e]);
         }
 #pragma unroll
         for (int k = 0; k < BS; ++k) piv[int64_t(i) * BS + k] = pv[k];
@@ -289,12 +288,10 @@ __global__ void __launch_bounds__(kLuThreads, BS == 6 ? 3 : 4) k_lu(BsrView A, c
         }
     }
     __syncthreads();
-    const int64_t base = int64_t(r0) * B2;
+    MT* dst = lu + int64_t(r0) * B2;
     for (int q = threadIdx.x; q < nrows * B2; q += kLuThreads) {
         const int row = q / B2, e = q - row * B2;
-        const double o = sm[row * SP + e];
-        if (lu) lu[base + q] = static_cast<MT>(o);
-        if (INV && inv64) inv64[base + q] = o;
+        dst[q] = sm[row * SP + e];
     }
 }
 
@@ -1026,12 +1023,12 @@ void launch_spmv_ex(const BsrView& A, const MT* vals, const double* x, double* y
 }
 
 template <typename MT>
-void launch_lu_setup(const BsrView& A, const MT* vals, MT* lu, double* inv64, int8_t* piv, int* err_flag,
-                     bool inverse, cudaStream_t s) {
+void launch_lu_setup(const BsrView& A, const MT* vals, MT* lu, int8_t* piv, int* err_flag, bool inverse,
+                     cudaStream_t s) {
     const unsigned gr = grid_for(A.n, kLuThreads);
 #define CFDG_LU(BS)                                                                          \
-    if (inverse) launch_after(k_lu<MT, BS, true>, gr, kLuThreads, 0, s, A, vals, lu, inv64, piv, err_flag); \
-    else launch_after(k_lu<MT, BS, false>, gr, kLuThreads, 0, s, A, vals, lu, inv64, piv, err_flag)
+    if (inverse) launch_after(k_lu<MT, BS, true>, gr, kLuThreads, 0, s, A, vals, lu, piv, err_flag); \
+    else launch_after(k_lu<MT, BS, false>, gr, kLuThreads, 0, s, A, vals, lu, piv, err_flag)
     switch (A.bs) {
         case 1: CFDG_LU(1); break;
         case 3: CFDG_LU(3); break;
@@ -1260,9 +1257,8 @@ template void launch_sgs_last_spmv<double>(const BsrView&, const double*, const 
                                            const DotSpec&, double*, const int*, cudaStream_t);
 template void launch_sgs_last_spmv<float>(const BsrView&, const float*, const float*, int32_t, double*, double*,
                                           const DotSpec&, double*, const int*, cudaStream_t);
-template void launch_lu_setup<double>(const BsrView&, const double*, double*, double*, int8_t*, int*, bool,
-                                      cudaStream_t);
-template void launch_lu_setup<float>(const BsrView&, const float*, float*, double*, int8_t*, int*, bool, cudaStream_t);
+template void launch_lu_setup<double>(const BsrView&, const double*, double*, int8_t*, int*, bool, cudaStream_t);
+template void launch_lu_setup<float>(const BsrView&, const float*, float*, int8_t*, int*, bool, cudaStream_t);
 template bool launch_sgs_level_coop<double>(const BsrView&, const double*, const double*, const int8_t*,
                                             const int4*, const int32_t*, int, const int4*, const int32_t*, int,
                                             const double*, double*, const int*, cudaStream_t);

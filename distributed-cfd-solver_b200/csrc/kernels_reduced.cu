@@ -17,8 +17,8 @@
 // only, and x_0 follows at the end from its own rows,
 //     x_0 = D_0^-1 (b_0 - cr rho_0 - U x_R).
 // The iterates are those of BiCGSTAB::solve (src/linalg/bicgstab.cpp:42-201)
-// on the full system; only rounding differs.  D^-1 is FP64 also for the FP32
-// matrix: the product relies on D D^-1 = I, which FP32 factors would hold
+// on the full system; only rounding differs.  FP64 matrices only: the product
+// relies on D D^-1 = I, which the FP32 inverse of a mixed-precision system holds
 // only to 1e-7.
 //
 // All passes are bound by the matrix and vector traffic; the reductions end in
@@ -32,41 +32,37 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int64_t kGridCap = 148 * 8;  // resident 256-thread blocks; bounds the partials a last block reads
 
-template <typename MT>
-__device__ __forceinline__ double ldv(const MT* p) { return static_cast<double>(__ldg(p)); }
-
 // BS consecutive entries at p (matrix block row or vector block); 6 and 4
 // entries start on pair boundaries and load as pairs.
-template <typename T, int BS>
-__device__ __forceinline__ void load_row(const T* p, double (&out)[BS]) {
+template <int BS>
+__device__ __forceinline__ void load_row(const double* p, double (&out)[BS]) {
     if constexpr (BS == 6 || BS == 4) {
-        using P = typename std::conditional<sizeof(T) == 8, double2, float2>::type;
-        const P* q = reinterpret_cast<const P*>(p);
+        const double2* q = reinterpret_cast<const double2*>(p);
 #pragma unroll
         for (int h = 0; h < BS / 2; ++h) {
-            const P v = __ldg(q + h);
+            const double2 v = __ldg(q + h);
             out[2 * h] = v.x;
             out[2 * h + 1] = v.y;
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < BS; ++j) out[j] = ldv(p + j);
+        for (int j = 0; j < BS; ++j) out[j] = __ldg(p + j);
     }
 }
 
 // sum over blocks [k0, k1) (skipping block `skip`) of A_k[ii][:] . x_col(k);
 // PAIRS: x is 16-byte aligned (the system's own vectors; a caller's may not be)
-template <typename MT, int BS, bool PAIRS = true>
-__device__ __forceinline__ double row_sum(const RedView& A, const MT* __restrict__ vals, const double* x, int ii,
+template <int BS, bool PAIRS = true>
+__device__ __forceinline__ double row_sum(const RedView& A, const double* __restrict__ vals, const double* x, int ii,
                                           int32_t k0, int32_t k1, int32_t skip) {
     double acc = 0.0;
     for (int32_t k = k0; k < k1; ++k) {
         if (k == skip) continue;
         double a[BS], xb[BS];
-        load_row<MT, BS>(vals + int64_t(k) * (BS * BS) + ii * BS, a);
+        load_row<BS>(vals + int64_t(k) * (BS * BS) + ii * BS, a);
         const double* xk = x + int64_t(__ldg(A.cols + k)) * BS;
         if constexpr (PAIRS) {
-            load_row<double, BS>(xk, xb);
+            load_row<BS>(xk, xb);
         } else {
 #pragma unroll
             for (int j = 0; j < BS; ++j) xb[j] = xk[j];
@@ -90,7 +86,7 @@ __device__ __forceinline__ double apply_dinv(const double* __restrict__ dinv, in
     double out = 0.0;
     if (act) {
         double d[BS];
-        load_row<double, BS>(dinv + int64_t(i) * (BS * BS) + ii * BS, d);
+        load_row<BS>(dinv + int64_t(i) * (BS * BS) + ii * BS, d);
 #pragma unroll
         for (int j = 0; j < BS; ++j) out += d[j] * b[j];
     }
@@ -242,9 +238,9 @@ __global__ void __launch_bounds__(kThreads) k_red_guess_reset(RedView A, const K
 // block are independent loads, and a row's blocks follow one another.
 enum { BACK0, BACK, FWD, ETA, WSUM, XRED };
 
-template <typename MT, int BS, bool LIST, int KIND>
+template <int BS, bool LIST, int KIND>
 __global__ void __launch_bounds__(kThreads, BS <= 5 ? 8 : 6)
-    k_red_sweep(RedView A, const MT* __restrict__ vals, const double* __restrict__ dinv, int32_t pos0, int32_t pos1,
+    k_red_sweep(RedView A, const double* __restrict__ vals, const double* __restrict__ dinv, int32_t pos0, int32_t pos1,
                 const double* src, const double* w, double* z, double* e, const KrylovScalars* __restrict__ ks,
                 int second) {
     if (KIND == XRED ? ks->updates == 0 : ks->state != KS_RUNNING) return;
@@ -258,20 +254,20 @@ __global__ void __launch_bounds__(kThreads, BS <= 5 ? 8 : 6)
         const int64_t t = int64_t(i) * BS + L.ii;
         const int32_t d = A.diag[i];
         if (KIND == BACK0 || KIND == BACK) {
-            s = row_sum<MT, BS>(A, vals, z, L.ii, LIST ? A.row_ptr[i] : d + 1, A.row_ptr[i + 1], d);
+            s = row_sum<BS>(A, vals, z, L.ii, LIST ? A.row_ptr[i] : d + 1, A.row_ptr[i + 1], d);
         } else if (KIND == FWD) {
             const double c = second ? ks->cs : ks->cp;
             s = src[t] - c * w[t];
-            if (!LIST) s -= row_sum<MT, BS>(A, vals, z, L.ii, A.mid[i], d, d);  // a list has two colours: no mid
+            if (!LIST) s -= row_sum<BS>(A, vals, z, L.ii, A.mid[i], d, d);  // a list has two colours: no mid
         } else if (KIND == ETA) {
             s = src[t];
         } else if (KIND == WSUM) {
-            s = LIST ? row_sum<MT, BS>(A, vals, e, L.ii, A.row_ptr[i], A.row_ptr[i + 1], d)
-                     : row_sum<MT, BS>(A, vals, e, L.ii, A.row_ptr[i], A.mid[i], d);
+            s = LIST ? row_sum<BS>(A, vals, e, L.ii, A.row_ptr[i], A.row_ptr[i + 1], d)
+                     : row_sum<BS>(A, vals, e, L.ii, A.row_ptr[i], A.mid[i], d);
         } else {
             const double* x = ks->x;
             s = ks->b[t] - ks->cr * src[t];
-            s -= row_sum<MT, BS, false>(A, vals, x, L.ii, LIST ? A.row_ptr[i] : d + 1, A.row_ptr[i + 1], d);
+            s -= row_sum<BS, false>(A, vals, x, L.ii, LIST ? A.row_ptr[i] : d + 1, A.row_ptr[i + 1], d);
         }
     }
     if constexpr (KIND == WSUM) {
@@ -295,9 +291,9 @@ __global__ void __launch_bounds__(kThreads, BS <= 5 ? 8 : 6)
 // FIRST (v = A M^-1 p): gamma = r0.v -> alpha, and s_0 = cs rho_0;
 // else (t = A M^-1 s): the five products -> omega, |r|, rho and beta
 // (bicgstab.cpp:112-158) with the colour-0 parts from the scalars.
-template <typename MT, int BS, bool LIST, bool FIRST>
+template <int BS, bool LIST, bool FIRST>
 __global__ void __launch_bounds__(kThreads, BS <= 5 ? 6 : 5)
-    k_red_product(RedView A, const MT* __restrict__ vals, const double* __restrict__ src, const double* __restrict__ e,
+    k_red_product(RedView A, const double* __restrict__ vals, const double* __restrict__ src, const double* __restrict__ e,
                   double* __restrict__ out, const double* __restrict__ r0, KrylovScalars* ks,
                   double* __restrict__ partials) {
     if (ks->state != KS_RUNNING) return;
@@ -314,7 +310,7 @@ __global__ void __launch_bounds__(kThreads, BS <= 5 ? 6 : 5)
         const int64_t t = int64_t(i) * BS + L.ii;
         const int32_t d = A.diag[i];
         const double sv = src[t];
-        const double o = sv - row_sum<MT, BS>(A, vals, e, L.ii, A.row_ptr[i], LIST ? A.row_ptr[i + 1] : d, d);
+        const double o = sv - row_sum<BS>(A, vals, e, L.ii, A.row_ptr[i], LIST ? A.row_ptr[i + 1] : d, d);
         out[t] = o;
         const double q = r0[t];
         if constexpr (FIRST) {
@@ -506,8 +502,7 @@ void launch_red_init(const RedView& A, KrylovScalars* ks, const double* v, doubl
     });
 }
 
-template <typename MT>
-void launch_red_sweep(const RedView& A, const MT* vals, const double* dinv, int kind, int32_t pos0, int32_t pos1,
+void launch_red_sweep(const RedView& A, const double* vals, const double* dinv, int kind, int32_t pos0, int32_t pos1,
                       const double* src, const double* w, double* z, double* e, const KrylovScalars* ks, bool second,
                       cudaStream_t st) {
     if (pos1 <= pos0) return;
@@ -515,7 +510,7 @@ void launch_red_sweep(const RedView& A, const MT* vals, const double* dinv, int 
         constexpr int BS = decltype(c)::value;
         const unsigned g = capped_grid<BS>(pos1 - pos0, int64_t(1) << 31);
         auto go = [&](auto list, auto k) {
-            k_red_sweep<MT, BS, decltype(list)::value, decltype(k)::value>
+            k_red_sweep<BS, decltype(list)::value, decltype(k)::value>
                 <<<g, kThreads, 0, st>>>(A, vals, dinv, pos0, pos1, src, w, z, e, ks, second ? 1 : 0);
         };
         auto by_list = [&](auto k) {
@@ -533,15 +528,14 @@ void launch_red_sweep(const RedView& A, const MT* vals, const double* dinv, int 
     });
 }
 
-template <typename MT>
-void launch_red_product(const RedView& A, const MT* vals, const double* src, const double* e, double* out,
+void launch_red_product(const RedView& A, const double* vals, const double* src, const double* e, double* out,
                         const double* r0, KrylovScalars* ks, double* partials, bool first, cudaStream_t st) {
     by_block_size(A.bs, [&](auto c) {
         constexpr int BS = decltype(c)::value;
         // exactly the resident blocks of the launch bounds
         const unsigned g = capped_grid<BS>(A.n - A.n0, 148 * (BS <= 5 ? 6 : 5));
         auto go = [&](auto list, auto f) {
-            k_red_product<MT, BS, decltype(list)::value, decltype(f)::value>
+            k_red_product<BS, decltype(list)::value, decltype(f)::value>
                 <<<g, kThreads, 0, st>>>(A, vals, src, e, out, r0, ks, partials);
         };
         if (A.rows) first ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
@@ -570,16 +564,5 @@ void launch_red_update(const RedView& A, const double* dinv, const double* zs, c
 void launch_red_enter(const KrylovScalars* ks, cudaGraphConditionalHandle cond, cudaStream_t st) {
     k_red_enter<<<1, 32, 0, st>>>(ks, cond);
 }
-
-template void launch_red_sweep<double>(const RedView&, const double*, const double*, int, int32_t, int32_t,
-                                       const double*, const double*, double*, double*, const KrylovScalars*, bool,
-                                       cudaStream_t);
-template void launch_red_sweep<float>(const RedView&, const float*, const double*, int, int32_t, int32_t,
-                                      const double*, const double*, double*, double*, const KrylovScalars*, bool,
-                                      cudaStream_t);
-template void launch_red_product<double>(const RedView&, const double*, const double*, const double*, double*,
-                                         const double*, KrylovScalars*, double*, bool, cudaStream_t);
-template void launch_red_product<float>(const RedView&, const float*, const double*, const double*, double*,
-                                        const double*, KrylovScalars*, double*, bool, cudaStream_t);
 
 }  // namespace cfdg

@@ -48,12 +48,10 @@ void launch_red_init(const RedView& A, KrylovScalars* ks, const double* v, doubl
                      double* partials, bool guess, cudaStream_t st);
 // One sweep pass over the positions [pos0, pos1); second: the s vector's
 // sweep (cs), else the p vector's (cp)
-template <typename MT>
-void launch_red_sweep(const RedView& A, const MT* vals, const double* dinv, int kind, int32_t pos0, int32_t pos1,
+void launch_red_sweep(const RedView& A, const double* vals, const double* dinv, int kind, int32_t pos0, int32_t pos1,
                       const double* src, const double* w, double* z, double* e, const KrylovScalars* ks, bool second,
                       cudaStream_t st);
-template <typename MT>
-void launch_red_product(const RedView& A, const MT* vals, const double* src, const double* e, double* out,
+void launch_red_product(const RedView& A, const double* vals, const double* src, const double* e, double* out,
                         const double* r0, KrylovScalars* ks, double* partials, bool first, cudaStream_t st);
 void launch_red_s(const RedView& A, const double* dinv, const double* r, const double* v, const double* w, double* s,
                   double* z, const KrylovScalars* ks, cudaStream_t st);

@@ -289,7 +289,6 @@ void BsrSystem::set_precision(int precision) {
     } else {
         vals32_.release();
         lu32_.release();
-        dinv64_.release();
         alloc_or_throw(vals64_, nv, "values");
     }
     precision_ = precision;
@@ -450,7 +449,7 @@ void BsrSystem::build_ordering(int ordering) {
     // colour order, or two colours, where every off-diagonal block of a row
     // is of the other colour.
     const int ncolor = static_cast<int>(fwd_off_.size()) - 1;
-    reducible_ = reduce != REDUCE_NONE && ordering == CFDG_SGS_COLOR && ncolor >= 2 && (split_ || ncolor == 2);
+    reducible_ = reduce && ordering == CFDG_SGS_COLOR && ncolor >= 2 && (split_ || ncolor == 2);
     if (reducible_) {
         std::vector<int32_t> mid(n);
         for (int32_t i = 0; i < n; ++i) {
@@ -608,15 +607,13 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
     const bool color = ordering_ == CFDG_SGS_COLOR;
     const double b2 = double(bs_) * bs_;
     if (precision_ == CFDG_PREC_MIXED) {
-        const bool inv64 = color && reducible();
         if (!lu32_.p && n_ > 0) alloc_or_throw(lu32_, nb2, "lu");
-        if (inv64 && !dinv64_.p) alloc_or_throw(dinv64_, nb2, "diagonal inverses");
-        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * (8.0 + (inv64 ? 8.0 : 0.0)) + bs_ + 4.0));
-        launch_lu_setup<float>(view(), vals32_.p, lu32_.p, inv64 ? dinv64_.p : nullptr, piv_.p, err_.p, color, stream_);
+        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 8.0 + bs_ + 4.0));
+        launch_lu_setup<float>(view(), vals32_.p, lu32_.p, piv_.p, err_.p, color, stream_);
     } else {
         if (!lu64_.p && n_ > 0) alloc_or_throw(lu64_, nb2, "lu");
         ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + bs_ + 4.0));
-        launch_lu_setup<double>(view(), vals64_.p, lu64_.p, nullptr, piv_.p, err_.p, color, stream_);
+        launch_lu_setup<double>(view(), vals64_.p, lu64_.p, piv_.p, err_.p, color, stream_);
     }
     cuda_check(cudaGetLastError(), "lu launch");
     const bool was = sell_on_;
@@ -993,8 +990,7 @@ double BsrSystem::red_bytes(const PassCount& c, double dinv_rows, double vectors
 
 // r = b - A x (the product already in v_ unless x = 0), w, and the first
 // step of the first sweep.
-template <typename MT>
-void BsrSystem::red_begin_t(const MT* vals, const double* dinv, Start start) {
+void BsrSystem::red_begin(Start start) {
     const RedView R = red_view();
     const double N = double(n_) * bs_, n0 = R.n0;
     {
@@ -1007,64 +1003,59 @@ void BsrSystem::red_begin_t(const MT* vals, const double* dinv, Start start) {
         ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 3,
                      n0 * bs_ * (bs_ * 8.0 + 16.0) + red_bytes(red_w_, 0.0, 1.0) +
                          red_bytes(PassCount{red_fwd_[1].rows, 0.0, 0.0}, red_fwd_[1].rows, 3.0));
-        launch_red_sweep<MT>(R, vals, dinv, RED_ETA, 0, R.n0, r0_.p, nullptr, nullptr, t_.p, ks_.p, false, stream_);
-        launch_red_sweep<MT>(R, vals, dinv, RED_WSUM, R.n0, n_, nullptr, nullptr, w_.p, t_.p, ks_.p, false, stream_);
-        launch_red_sweep<MT>(R, vals, dinv, RED_FWD, R.n0, R.n1, p_.p, w_.p, phat_.p, nullptr, ks_.p, false, stream_);
+        const double *vals = vals64_.p, *dinv = lu64_.p;
+        launch_red_sweep(R, vals, dinv, RED_ETA, 0, R.n0, r0_.p, nullptr, nullptr, t_.p, ks_.p, false, stream_);
+        launch_red_sweep(R, vals, dinv, RED_WSUM, R.n0, n_, nullptr, nullptr, w_.p, t_.p, ks_.p, false, stream_);
+        launch_red_sweep(R, vals, dinv, RED_FWD, R.n0, R.n1, p_.p, w_.p, phat_.p, nullptr, ks_.p, false, stream_);
     }
 }
 
 // out = A M^-1 src on the rest rows with the inner products; z holds the
 // sweep of colour 1 on entry and M^-1 src (rest rows) on return, e = D^-1 U z.
-template <typename MT>
-void BsrSystem::red_apply_t(const MT* vals, const double* dinv, const double* src, double* z, double* e, double* out,
-                            bool second) {
+void BsrSystem::red_apply(const double* src, double* z, double* e, double* out, bool second) {
     const RedView R = red_view();
     const int ng = groups_fwd();
     auto pass = [&](int kind, int g, const PassCount& c, double vectors) {
         ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, red_bytes(c, c.rows, vectors));
-        launch_red_sweep<MT>(R, vals, dinv, kind, fwd_off_[g], fwd_off_[g + 1], src, w_.p, z, e, ks_.p, second,
+        launch_red_sweep(R, vals64_.p, lu64_.p, kind, fwd_off_[g], fwd_off_[g + 1], src, w_.p, z, e, ks_.p, second,
                              stream_);
     };
     for (int g = 2; g < ng; ++g) pass(RED_FWD, g, red_fwd_[g], 3.0);
     for (int g = ng - 2; g >= 1; --g) pass(RED_BACK, g, red_back_[g], 3.0);
     pass(RED_BACK0, 0, red_back_[0], 1.0);
     ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, red_bytes(red_lower_, 0.0, 3.0));
-    launch_red_product<MT>(R, vals, src, e, out, r0_.p, ks_.p, partials_.p, !second, stream_);
+    launch_red_product(R, vals64_.p, src, e, out, r0_.p, ks_.p, partials_.p, !second, stream_);
 }
 
 // One BiCGSTAB iteration (bicgstab.cpp:84-176); every kernel is gated by the
 // device-side state.  e of the first product lies in t (written by the
 // second), e of the second in r (rewritten by the update).
-template <typename MT>
-void BsrSystem::red_iteration_t(const MT* vals, const double* dinv, bool use_cond) {
+void BsrSystem::red_iteration(bool use_cond) {
     const RedView R = red_view();
     const double rest = double(n_ - R.n0) * bs_ * 8.0, c1 = double(R.n1 - R.n0) * bs_;
-    red_apply_t<MT>(vals, dinv, p_.p, phat_.p, t_.p, v_.p, false);
+    red_apply(p_.p, phat_.p, t_.p, v_.p, false);
     {
         ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 3.0 * rest + c1 * (bs_ * 8.0 + 16.0));
-        launch_red_s(R, dinv, r_.p, v_.p, w_.p, s_.p, shat_.p, ks_.p, stream_);
+        launch_red_s(R, lu64_.p, r_.p, v_.p, w_.p, s_.p, shat_.p, ks_.p, stream_);
     }
-    red_apply_t<MT>(vals, dinv, s_.p, shat_.p, r_.p, t_.p, true);
+    red_apply(s_.p, shat_.p, r_.p, t_.p, true);
     ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 1, 10.0 * rest + c1 * (bs_ * 8.0 + 16.0));
-    launch_red_update(R, dinv, shat_.p, s_.p, t_.p, v_.p, w_.p, r_.p, p_.p, phat_.p, ks_.p, partials_.p, loop_handle_,
+    launch_red_update(R, lu64_.p, shat_.p, s_.p, t_.p, v_.p, w_.p, r_.p, p_.p, phat_.p, ks_.p, partials_.p, loop_handle_,
                       use_cond, stream_);
 }
 
 // x on colour 0 from its own rows.
-template <typename MT>
-void BsrSystem::red_end_t(const MT* vals, const double* dinv) {
+void BsrSystem::red_end() {
     ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, red_bytes(red_back_[0], red_back_[0].rows, 3.0));
-    launch_red_sweep<MT>(red_view(), vals, dinv, RED_XRED, 0, fwd_off_[1], r0_.p, nullptr, nullptr, nullptr, ks_.p,
-                         false, stream_);
+    launch_red_sweep(red_view(), vals64_.p, lu64_.p, RED_XRED, 0, fwd_off_[1], r0_.p, nullptr, nullptr, nullptr, ks_.p,
+                     false, stream_);
 }
 
 // The whole solve as one graph: [begin] -> while [iteration] -> [end].  An
 // error on the way leaves the host loop in charge.
 bool BsrSystem::red_graph_ready(Start start) {
-    if (red_exec_precision_ != precision_) release_red_graphs();
     if (red_exec_[start]) return true;
     if (loop_failed_) return false;
-    const bool mixed = precision_ == CFDG_PREC_MIXED;
     const int64_t launches0 = prof_->launches;
     cudaGraph_t g = nullptr;
     bool capturing = false;
@@ -1082,8 +1073,7 @@ bool BsrSystem::red_graph_ready(Start start) {
         cuda_check(cudaGraphCreate(&g, 0), "graph create");
         cuda_check(cudaGraphConditionalHandleCreate(&loop_handle_, g, 0, cudaGraphCondAssignDefault), "graph handle");
         begin_capture(g, nullptr, 0);
-        if (mixed) red_begin_t<float>(vals32_.p, dinv(), start);
-        else red_begin_t<double>(vals64_.p, dinv(), start);
+        red_begin(start);
         launch_red_enter(ks_.p, loop_handle_, stream_);
         ++prof_->launches;
         cudaStreamCaptureStatus status;
@@ -1101,13 +1091,11 @@ bool BsrSystem::red_graph_ready(Start start) {
         cuda_check(cudaGraphAddNode(&loop, g, before.data(), before.size(), &cp), "graph conditional node");
         const int64_t l1 = prof_->launches;
         begin_capture(cp.conditional.phGraph_out[0], nullptr, 0);
-        if (mixed) red_iteration_t<float>(vals32_.p, dinv(), true);
-        else red_iteration_t<double>(vals64_.p, dinv(), true);
+        red_iteration(true);
         end_capture();
         red_body_launches_ = prof_->launches - l1;
         begin_capture(g, &loop, 1);
-        if (mixed) red_end_t<float>(vals32_.p, dinv());
-        else red_end_t<double>(vals64_.p, dinv());
+        red_end();
         end_capture();
         cuda_check(cudaGetLastError(), "graph capture");
         cuda_check(cudaGraphInstantiate(&red_exec_[start], g, 0), "graph instantiate");
@@ -1123,7 +1111,6 @@ bool BsrSystem::red_graph_ready(Start start) {
     red_fixed_launches_[start] = prof_->launches - launches0 - red_body_launches_;
     prof_->launches = launches0;
     if (g) cudaGraphDestroy(g);
-    red_exec_precision_ = precision_;
     return red_exec_[start] != nullptr;
 }
 
@@ -1136,7 +1123,6 @@ void BsrSystem::release_red_graphs() {
 
 cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, int max_it, double* x, const double* b,
                                                Start start) {
-    const bool mixed = precision_ == CFDG_PREC_MIXED;
     *ks_init_ = KrylovScalars{};
     ks_init_->max_it = max_it;
     ks_init_->rel_tol = rel_tol;
@@ -1148,8 +1134,7 @@ cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, i
     if (start != START_ZERO) {
         DotSpec none{};
         ProfScope ps(prof_, CFDG_KCAT_SPMV, stream_, 1, spmv_bytes(0, false));
-        if (mixed) launch_spmv_ex<float>(view(), vals32_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
-        else launch_spmv_ex<double>(view(), vals64_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
+        launch_spmv_ex<double>(view(), vals64_.p, x, v_.p, 1.0, 0.0, none, nullptr, nullptr, stream_);
     }
     auto read = [&] { read_scalars(); };
     if (device_loop && !prof_->on() && red_graph_ready(start)) {
@@ -1157,21 +1142,18 @@ cfdg_krylov_result BsrSystem::bicgstab_reduced(double rel_tol, double abs_tol, i
         read();
         prof_->launches += red_fixed_launches_[start] + red_body_launches_ * ks_host_->body_runs;
     } else {
-        if (mixed) red_begin_t<float>(vals32_.p, dinv(), start);
-        else red_begin_t<double>(vals64_.p, dinv(), start);
+        red_begin(start);
         int it = 0;
         bool done = false;
         while (!done && it < max_it) {
-            if (mixed) red_iteration_t<float>(vals32_.p, dinv(), false);
-            else red_iteration_t<double>(vals64_.p, dinv(), false);
+            red_iteration(false);
             ++it;
             if (it % check_every == 0 || it == max_it) {
                 read();
                 if (ks_host_->state != KS_RUNNING) done = true;
             }
         }
-        if (mixed) red_end_t<float>(vals32_.p, dinv());
-        else red_end_t<double>(vals64_.p, dinv());
+        red_end();
         cuda_check(cudaGetLastError(), "krylov launch");
         read();
     }
@@ -1910,12 +1892,10 @@ void Solver::setup_matrix(const HostMesh& hm, const Csr& c2c) {
     // the wall-stretched viscous systems an unconverged solve amplifies
     // rounding up to 1e13 times (two solves whose input differs by one unit in
     // the last place end 1e-3 apart on the Spalart-Allmaras plate, 30
-    // iterations), and its FP64 D^-1 is another preconditioner than the
-    // FP32-rounded one of a mixed-precision solve (the supersonic ramp moves by
-    // 1e-6 in three steps): there the full solve stays.  Inviscid FP64 solves
-    // agree to 1e-12, and are 1.2x faster (4,096-cell ramp, ten steady
+    // iterations): there the full solve stays.  Inviscid FP64 solves agree to
+    // 1e-12, and are 1.2x faster (4,096-cell ramp, ten steady
     // iterations: 2.91 -> 2.41 ms).
-    sys_->reduce = cfg_.viscous ? BsrSystem::REDUCE_NONE : BsrSystem::REDUCE_FP64;
+    sys_->reduce = cfg_.viscous == 0;
     auto pos = [&](int32_t row, int32_t col) -> int32_t {
         const auto b = cols.begin() + row_ptr[row], e = cols.begin() + row_ptr[row + 1];
         const auto it = std::lower_bound(b, e, col);

@@ -191,11 +191,8 @@ public:
     void set_product(Product p) { product_ = std::move(p); }
     int check_every = 1;  // host loop: polls the Krylov state every k iterations
     bool device_loop = true;  // run the iterations as one graph launch (CFDG_KRYLOV_DEVICE_LOOP)
-    // Systems whose multicolour BiCGSTAB runs in its reduced form
-    // (kernels_reduced.cu).
     bool sliced = false;  // keep a sliced copy of the matrix where that pays (the owner refills the values each solve)
-    enum Reduce { REDUCE_NONE, REDUCE_FP64, REDUCE_ANY };
-    Reduce reduce = REDUCE_ANY;
+    bool reduce = true;   // run the multicolour BiCGSTAB of FP64 systems in its reduced form (kernels_reduced.cu)
 
 private:
     void build_ordering(int ordering);
@@ -226,19 +223,14 @@ private:
     // BiCGSTAB + one multicolour sweep on the rows outside the first colour
     // (kernels_reduced.cu)
     bool reducible() const {
-        return reducible_ && sweeps_ == 1 && (reduce == REDUCE_ANY || (reduce == REDUCE_FP64 && precision_ == CFDG_PREC_FP64));
+        return reducible_ && sweeps_ == 1 && precision_ == CFDG_PREC_FP64;
     }
     cfdg_krylov_result bicgstab_reduced(double rel_tol, double abs_tol, int max_it, double* x, const double* b,
                                         Start start);
-    template <typename MT>
-    void red_begin_t(const MT* vals, const double* dinv, Start start);
-    template <typename MT>
-    void red_iteration_t(const MT* vals, const double* dinv, bool use_cond);
-    template <typename MT>
-    void red_apply_t(const MT* vals, const double* dinv, const double* src, double* z, double* e, double* out,
-                     bool second);
-    template <typename MT>
-    void red_end_t(const MT* vals, const double* dinv);
+    void red_begin(Start start);
+    void red_iteration(bool use_cond);
+    void red_apply(const double* src, double* z, double* e, double* out, bool second);
+    void red_end();
     bool red_graph_ready(Start start);
     void release_red_graphs();
     cfdg_krylov_result krylov_result() const;
@@ -280,7 +272,7 @@ private:
     // or have two colours; blocks and distinct vector entries its passes read
     bool reducible_ = false;
     DevArray<int32_t> mid_;    // first block of a row outside the colour-0 columns
-    DevArray<double> w_, dinv64_;
+    DevArray<double> w_;
     struct PassCount {
         double rows = 0.0, blocks = 0.0, entries = 0.0;
     };
@@ -288,12 +280,10 @@ private:
     PassCount red_lower_, red_w_;
     double red_bytes(const PassCount& c, double dinv_rows, double vectors) const;
     RedView red_view() const;
-    const double* dinv() const { return precision_ == CFDG_PREC_MIXED ? dinv64_.p : lu64_.p; }
     // [start]: initial residual and w, the iterations as a conditional
     // while-node, and x on colour 0, on the system's own buffers (the
     // caller's x and b are read through the device scalars)
     cudaGraphExec_t red_exec_[3] = {nullptr, nullptr, nullptr};
-    int red_exec_precision_ = -1;
     int64_t red_fixed_launches_[3] = {0, 0, 0}, red_body_launches_ = 0;
     KrylovScalars* ks_init_ = nullptr;  // pinned: the scalars a solve starts from
     // rows [fwd_off_[1], n) of a colour-ordered matrix: block count and

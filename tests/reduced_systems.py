@@ -68,12 +68,25 @@ def dense(row_ptr, cols, vals, bs):
     return M
 
 
-def colour_sgs(M, colour, bs):
-    """z = M^-1 r of one symmetric sweep in colour order, dense."""
+def colour_sgs(M, colour, bs, fp32=False):
+    """z = M^-1 r of one symmetric sweep in colour order, dense; fp32: with the
+    diagonal inverses of a mixed-precision system, rounded to FP32."""
     c = np.repeat(colour, bs)
     unit = np.repeat(np.arange(len(colour)), bs)
     same = unit[:, None] == unit[None, :]
     low = np.where((c[None, :] < c[:, None]) & ~same, M, 0.0)
     up = np.where((c[None, :] > c[:, None]) & ~same, M, 0.0)
     D = np.where(same, M, 0.0)
-    return lambda r: np.linalg.solve(D + up, D @ np.linalg.solve(D + low, r))
+    if not fp32:
+        return lambda r: np.linalg.solve(D + up, D @ np.linalg.solve(D + low, r))
+    inv = np.linalg.inv(D).astype(np.float32).astype(np.float64)
+
+    def apply(r):
+        z = np.zeros_like(r)
+        for g in range(colour.max() + 1):
+            z = np.where(c == g, inv @ (r - low @ z), z)
+        for g in range(colour.max(), -1, -1):
+            z = np.where(c == g, z - inv @ (up @ z), z)
+        return z
+
+    return apply
