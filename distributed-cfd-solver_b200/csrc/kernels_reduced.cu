@@ -17,9 +17,12 @@
 // only, and x_0 follows at the end from its own rows,
 //     x_0 = D_0^-1 (b_0 - cr rho_0 - U x_R).
 // The iterates are those of BiCGSTAB::solve (src/linalg/bicgstab.cpp:42-201)
-// on the full system; only rounding differs.  FP64 matrices only: the product
-// relies on D D^-1 = I, which the FP32 inverse of a mixed-precision system holds
-// only to 1e-7.
+// on the full system up to rounding, as far as D D^-1 = I holds: the product
+// does not multiply by D, so its error is that of D (D^-1 p) where the full
+// product's is that of A z.  k_red_check measures the difference for each
+// diagonal block, and the solve runs in the full form when one exceeds
+// kGrowthLimit.  FP64 matrices only: the FP32 inverse of a mixed-precision system
+// holds D D^-1 = I to 1e-7.
 //
 // All passes are bound by the matrix and vector traffic; the reductions end in
 // the last block of the kernel that forms them (one counter, fixed order),
@@ -469,6 +472,49 @@ __global__ void k_red_enter(const KrylovScalars* ks, cudaGraphConditionalHandle 
     if (threadIdx.x == 0) cudaGraphSetConditional(cond, ks->state == KS_RUNNING && ks->max_it > 0 ? 1u : 0u);
 }
 
+// Sets *flag when a diagonal block amplifies the rounding of the reduced
+// product.  With s = D v, the full product is wrong by about eps |D||v| and the
+// reduced one by eps |D||D^-1||s|, so in a norm that follows the scales of the
+// block's rows the loss is at most the norm of G = |D||D^-1|.  Scaled by a
+// positive x that norm is max_i (G x)_i / x_i, and three steps x <- G x bring it
+// close to its least value, the spectral radius: equations or variables in
+// other units change nothing (a transport Jacobian has 1.0 to 1.3 in SI units,
+// where cond(D) is 1e8), coupled stiff terms do.  Limit 8: on matrices whose blocks
+// have 4 to 8, both forms end at the same true residual, 2.6e-16 |b| (the worst
+// 1.25 times the other's); at 16 to 23 the reduced form ends at 1.7 times the
+// full one's, at 90 to 128 at 6 times, at 1e8 at 1e7 times.  Bound by the two
+// reads of n BS^2 values; a lane holds a row of both factors.
+constexpr double kGrowthLimit = 8.0;
+
+template <int BS>
+__global__ void __launch_bounds__(kThreads) k_red_check(RedView A, const double* vals, const double* dinv, int* flag) {
+    pdl_enter();
+    const Lanes<BS> L;
+    const int64_t i = warp_id() * L.GPW + L.grp;
+    const bool act = L.grp < L.GPW && i < A.n;
+    double d[BS], v[BS];
+    const double* dp = vals + (act ? int64_t(A.diag[i]) : 0) * (BS * BS) + L.ii * BS;
+    const double* vp = dinv + (act ? i : 0) * (BS * BS) + L.ii * BS;
+#pragma unroll
+    for (int j = 0; j < BS; ++j) {
+        d[j] = act ? fabs(dp[j]) : 0.0;
+        v[j] = act ? fabs(vp[j]) : 0.0;
+    }
+    auto times = [&](const double (&m)[BS], double x) {
+        double y = 0.0;
+#pragma unroll
+        for (int j = 0; j < BS; ++j) y += m[j] * __shfl_sync(0xffffffffu, x, L.base + j);
+        return y;
+    };
+    double x = 1.0, y = 1.0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x = y;
+        y = times(d, times(v, x));
+    }
+    if (act && !(y <= kGrowthLimit * x)) *flag = 1;  // not finite: over the limit too
+}
+
 template <int BS>
 unsigned capped_grid(int64_t rows, int64_t cap) {
     const int64_t warps = (rows + (32 / BS) - 1) / (32 / BS);
@@ -558,6 +604,13 @@ void launch_red_update(const RedView& A, const double* dinv, const double* zs, c
         constexpr int BS = decltype(c)::value;
         k_red_update<BS><<<capped_grid<BS>(A.n - A.n0, kGridCap), kThreads, 0, st>>>(
             A, dinv, zs, s, t, v, w, r, p, zp, ks, partials, cond, use_cond ? 1 : 0);
+    });
+}
+
+void launch_red_check(const RedView& A, const double* vals, const double* dinv, int* flag, cudaStream_t st) {
+    by_block_size(A.bs, [&](auto c) {
+        constexpr int BS = decltype(c)::value;
+        launch_after(k_red_check<BS>, capped_grid<BS>(A.n, int64_t(1) << 31), kThreads, 0, st, A, vals, dinv, flag);
     });
 }
 

@@ -43,6 +43,8 @@ struct RedView {
 };
 enum : int { RED_BACK0, RED_BACK, RED_FWD, RED_ETA, RED_WSUM, RED_XRED };
 int red_partials();  // doubles of the reduction buffer
+// *flag = 1 when a diagonal block would cost the reduced product accuracy
+void launch_red_check(const RedView& A, const double* vals, const double* dinv, int* flag, cudaStream_t st);
 // r0 = b - A x (v = A x; null: x = 0), r and p on the rest rows, the scalars
 void launch_red_init(const RedView& A, KrylovScalars* ks, const double* v, double* r, double* r0, double* p,
                      double* partials, bool guess, cudaStream_t st);

@@ -259,9 +259,9 @@ BsrSystem::BsrSystem(int device, int32_t n, int32_t bs, const int32_t* row_ptr, 
                             static_cast<std::size_t>(red_partials())) + 8,
                    "partials");
     alloc_or_throw(ks_, 1, "krylov scalars");
-    alloc_or_throw(err_, 1, "error flag");
+    alloc_or_throw(err_, 2, "error flags");
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_host_), sizeof(KrylovScalars)), "cudaMallocHost");
-    cuda_check(cudaMallocHost(reinterpret_cast<void**>(&err_host_), sizeof(int)), "cudaMallocHost");
+    cuda_check(cudaMallocHost(reinterpret_cast<void**>(&err_host_), 2 * sizeof(int)), "cudaMallocHost");
     cuda_check(cudaMallocHost(reinterpret_cast<void**>(&ks_init_), sizeof(KrylovScalars)), "cudaMallocHost");
 }
 
@@ -603,7 +603,7 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
     sweeps_ = sweeps;
     const std::size_t nb2 = static_cast<std::size_t>(n_) * bs_ * bs_;
     if (!piv_.p && n_ > 0) alloc_or_throw(piv_, static_cast<std::size_t>(n_) * bs_, "pivots");
-    cuda_check(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_), "memset");
+    cuda_check(cudaMemsetAsync(err_.p, 0, 2 * sizeof(int), stream_), "memset");
     const bool color = ordering_ == CFDG_SGS_COLOR;
     const double b2 = double(bs_) * bs_;
     if (precision_ == CFDG_PREC_MIXED) {
@@ -614,6 +614,10 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
         if (!lu64_.p && n_ > 0) alloc_or_throw(lu64_, nb2, "lu");
         ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + bs_ + 4.0));
         launch_lu_setup<double>(view(), vals64_.p, lu64_.p, piv_.p, err_.p, color, stream_);
+    }
+    if (reducible()) {
+        ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + 4.0));
+        launch_red_check(red_view(), vals64_.p, lu64_.p, err_.p + 1, stream_);
     }
     cuda_check(cudaGetLastError(), "lu launch");
     const bool was = sell_on_;
@@ -628,16 +632,17 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
     }
 }
 
-// Queues the copy of the factorisation's flag, if nobody has read it yet.
+// Queues the copy of the factorisation's flags, if nobody has read them yet.
 void BsrSystem::read_flag() {
     if (lu_unchecked_)
-        cuda_check(cudaMemcpyAsync(err_host_, err_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
+        cuda_check(cudaMemcpyAsync(err_host_, err_.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, stream_), "D2H");
 }
 
 void BsrSystem::check_factorisation() {
     if (!lu_unchecked_) return;
     lu_unchecked_ = false;
-    const int err = *err_host_;
+    lossy_ = err_host_[1] != 0;
+    const int err = err_host_[0];
     if (err == 0) return;
     lu_ready_ = false;
     if (err > 0)
@@ -1188,8 +1193,20 @@ cfdg_krylov_result BsrSystem::bicgstab(int precond, double rel_tol, double abs_t
                                        const double* b, Start start) {
     if (precond == CFDG_PC_SGS && !lu_ready_) throw Failure{CFDG_ERR_INVALID, "SGS preconditioner not set up"};
     const int64_t N = int64_t(n_) * bs_;
-    if (precond == CFDG_PC_SGS && !product_ && reducible())
-        return bicgstab_reduced(rel_tol, abs_tol, max_it, x, b, start);
+    if (precond == CFDG_PC_SGS && !product_ && reducible()) {
+        // Whether a diagonal block is lossy comes back with the solve's scalars
+        // when set-up did not wait for it; the flag is read first where the solve
+        // could not start again from zero, or the last set-up found one.
+        if (lu_unchecked_ && (lossy_ || start != START_ZERO)) {
+            read_flag();
+            cuda_check(cudaStreamSynchronize(stream_), "lu sync");
+            check_factorisation();
+        }
+        if (!lossy_) {
+            const cfdg_krylov_result res = bicgstab_reduced(rel_tol, abs_tol, max_it, x, b, start);
+            if (!lossy_) return res;
+        }
+    }
     const bool guess = start == START_GUESS;
     const BsrView A = view();
     const bool mixed = precision_ == CFDG_PREC_MIXED;

@@ -221,7 +221,7 @@ private:
     DevArray<double> sell64_, sellinv64_;
     DevArray<float> sell32_, sellinv32_;
     // BiCGSTAB + one multicolour sweep on the rows outside the first colour
-    // (kernels_reduced.cu)
+    // (kernels_reduced.cu), for matrices whose set-up found no lossy block
     bool reducible() const {
         return reducible_ && sweeps_ == 1 && precision_ == CFDG_PREC_FP64;
     }
@@ -249,8 +249,9 @@ private:
     DevArray<float> vals32_, lu32_;
     DevArray<int8_t> piv_;
     DevArray<int> err_;
-    int* err_host_ = nullptr;   // pinned copy of the factorisation's flag
+    int* err_host_ = nullptr;   // pinned copy of the factorisation's flags: failure, lossy block
     bool lu_unchecked_ = false; // ... which nobody has read yet
+    bool lossy_ = false;        // a diagonal block would cost the reduced solve accuracy
     int ordering_ = -1, sweeps_ = 1;
     int last_guess_ = 0;
     double last_bnorm_ = 0.0;

@@ -468,7 +468,13 @@ CFDG_API int cfdg_sgs_setup(cfdg_bsr* a, int32_t ordering, int32_t sweeps);
 CFDG_API int cfdg_sgs_apply(cfdg_bsr* a, const double* r_d, double* z_d);
 CFDG_API int cfdg_sgs_apply_host(cfdg_bsr* a, const double* r_h, double* z_h);
 /* IterativeSolver::solve for BiCGSTAB (src/linalg/bicgstab.cpp:42-201);
- * x holds the initial guess on entry.  precond: CFDG_PC_*. */
+ * x holds the initial guess on entry.  precond: CFDG_PC_*.
+ * An FP64 matrix with one CFDG_SGS_COLOR sweep and two colours or rows in
+ * colour order is solved on the rows outside the first colour: the same
+ * iterates, from two thirds of the matrix reads.  Rounding differs; set-up
+ * measures by how much for each diagonal block D (the norm of |D||D^-1| in
+ * the scales of its rows), and above 8 the solve takes the full form.  The
+ * reported residual is that of the recurrence, as in the reference. */
 CFDG_API int cfdg_bicgstab(cfdg_bsr* a, int32_t precond, double rel_tol, double abs_tol, int32_t max_it,
                   double* x_d, const double* b_d, cfdg_krylov_result* out_h);
 CFDG_API int cfdg_bicgstab_host(cfdg_bsr* a, int32_t precond, double rel_tol, double abs_tol, int32_t max_it,

@@ -173,3 +173,15 @@ def bicgstab_reduced(row_ptr, cols, vals, bs, colour, b, its, x0=None):
         rho = rho_new
     x0_rows = D(bb - cr * r0 - part(upper, np.where(rest[:, None], x, 0.0)))
     return np.where(zero[:, None], x0_rows, x).ravel()
+
+
+def growth(blocks):
+    """How much more rounding D (D^-1 s) takes than the product with D itself:
+    max_i (G x)_i / x_i of G = |D| |D^-1|, x after three steps x <- G x from ones
+    (an upper bound of the spectral radius of G, near it whatever the scales of
+    the block's rows and columns); per block."""
+    g = np.abs(blocks) @ np.abs(np.linalg.inv(blocks))
+    x = np.ones(blocks.shape[:2])
+    for _ in range(4):
+        x, old = np.einsum("kij,kj->ki", g, x), x
+    return (x / old).max(axis=1)

@@ -44,6 +44,22 @@ def system(kind, n, bs, order, seed=0):
     return row_ptr, cols, vals, colours(row_ptr, cols)
 
 
+def mix_equations(row_ptr, vals, bs, cond, seed=1):
+    """The system with each row's equations combined by a matrix of condition
+    `cond`: the same solution, diagonal blocks of that condition."""
+    rng = np.random.default_rng(seed)
+    n = len(row_ptr) - 1
+    q, p = (np.linalg.qr(rng.standard_normal((n, bs, bs)))[0] for _ in range(2))
+    t = np.einsum("kij,j,klj->kil", q, np.logspace(0.0, np.log10(cond), bs), p)
+    rows = np.repeat(np.arange(n), np.diff(row_ptr))
+    return np.einsum("kij,kjl->kil", t[rows], vals.reshape(-1, bs, bs)).ravel()
+
+
+def diagonal(row_ptr, cols, vals, bs):
+    rows = np.repeat(np.arange(len(row_ptr) - 1), np.diff(row_ptr))
+    return vals.reshape(-1, bs, bs)[rows == cols]
+
+
 def colours(row_ptr, cols):
     """The colours of the sweep: greedy over the row's columns and, where that
     leaves rows of a colour coupled, over the rows that list it too."""

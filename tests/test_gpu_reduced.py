@@ -55,3 +55,49 @@ def test_preconditioner_is_that_of_the_handle(cb, kind, n, bs, order, mixed):
     A.sgs_setup(cb.SGS_COLOR, 1)
     x, _ = A.bicgstab(b, rel_tol=1e-15, abs_tol=1e-300, max_it=1)
     assert rel_err(x, CS.bicgstab(A.spmv, A.sgs_apply, b, 1)) < 1e-10
+
+
+@pytest.mark.parametrize("kind,n,bs,order", [("box", 120, 5, "natural"), ("box", 121, 6, "colour"),
+                                             ("graph", 97, 3, "colour"), ("graph", 64, 4, "colour")])
+@pytest.mark.parametrize("cond", [1.0, 3.0, 10.0, 1e4, 1e7, 1e10])
+def test_converged_is_the_true_residual(cb, kind, n, bs, order, cond):
+    """Diagonal blocks on both sides of the limit on their growth: a solve that
+    reports convergence has reached its tolerance, and one run to the end reaches
+    what the full iteration in numpy does.  1.5e-15 |b|: four times the 2.2e-16 to
+    3.7e-16 that it ends at."""
+    rp, cl, vals, colour = RS.system(kind, n, bs, order)
+    vals = RS.mix_equations(rp, vals, bs, cond)
+    M = RS.dense(rp, cl, vals, bs)
+    b = M @ np.random.default_rng(3).standard_normal(n * bs)
+    A = cb.Bsr(rp, cl, bs)
+    A.set_values(vals)
+    A.sgs_setup(cb.SGS_COLOR, 1)
+    for tol in (1e-8, 1e-12):
+        x, info = A.bicgstab(b, rel_tol=tol, max_it=100)
+        assert info.status == cb.KRYLOV_CONVERGED
+        assert np.linalg.norm(b - M @ x) <= 1.01 * tol * np.linalg.norm(b)
+    x, _ = A.bicgstab(b, rel_tol=1e-30, abs_tol=1e-300, max_it=14)
+    assert np.linalg.norm(b - M @ x) < 1.5e-15 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("order", ["natural", "colour"])
+@pytest.mark.parametrize("cond", [1.0, 1e8])
+def test_long_solves(cb, order, cond):
+    """More than 32 iterations (the residual is formed from the vector every 32),
+    and the same handle on new values: the verdict is the matrix's."""
+    n, bs = 360, 5
+    rp, cl, vals, _ = RS.system("box", n, bs, order)
+    rows = np.repeat(np.arange(n), np.diff(rp))
+    v = vals.reshape(-1, bs, bs)
+    deg = np.diff(rp) - 1
+    v[rows == cl] += (0.7 * deg - 0.8 * (deg + 1) - 0.95)[:, None, None] * np.eye(bs)  # 48 iterations and more
+    A = cb.Bsr(rp, cl, bs)
+    for c in (1.0, cond):
+        w = RS.mix_equations(rp, vals, bs, c)
+        M = RS.dense(rp, cl, w, bs)
+        b = M @ np.random.default_rng(3).standard_normal(n * bs)
+        A.set_values(w)
+        A.sgs_setup(cb.SGS_COLOR, 1)
+        x, info = A.bicgstab(b, rel_tol=1e-10, max_it=500)
+        assert info.status == cb.KRYLOV_CONVERGED and info.iterations > 32
+        assert np.linalg.norm(b - M @ x) <= 1.01e-10 * np.linalg.norm(b)
