@@ -487,8 +487,8 @@ __global__ void __launch_bounds__(256) k_sgs_level_coop(BsrView A, const MT* __r
 // distributed shared memory (row i in CTA i mod C), the barrier is the
 // cluster's, and everything of a warp's next row that does not depend on z
 // (blocks, columns, r, LU factors, pivots) is loaded before the barrier.  One
-// cluster has the bandwidth for it: the levels of such a system hold a few
-// hundred rows.  The arithmetic of a row is k_sgs_level_coop's to the bit: one
+// cluster has the warps for levels of a few hundred rows; sgs_level_cluster
+// leaves systems with wider ones to the whole grid.  The arithmetic of a row is k_sgs_level_coop's to the bit: one
 // lane group per off-diagonal block, the products subtracted in ascending
 // column order, the pivoted substitution.  3.2 us a level on the same plate
 // (a sweep 0.96 -> 0.66 ms).
@@ -1149,11 +1149,30 @@ static int level_cluster(int32_t n, int* smem) {
     return 0;
 }
 
-int sgs_level_cluster(int32_t n, int bs, bool mixed, int* smem) {
-    if (n <= 0) return 0;
-    if (bs == 5) return mixed ? level_cluster<float, 5>(n, smem) : level_cluster<double, 5>(n, smem);
-    if (bs == 6) return mixed ? level_cluster<float, 6>(n, smem) : level_cluster<double, 6>(n, smem);
-    return 0;
+// The cluster takes the system where its sweep is the faster one.  A level costs
+// the cluster one turn of its warps (256 rows with 16 CTAs) per 256 rows begun,
+// 2.7 to 3.6 us each; the grid-wide sweep 5 us with hardly a dependence on the
+// width.  So the line is drawn on turns per level: measured (a sweep, grid-wide /
+// cluster, 5x5 FP64, boxes in row order and in colour order) 1,006 / 661 us at 1.0
+// turns (16k rows, 102 levels), 710 / 547 at 1.4, 2,690 / 2,306 at 1.8, 25 / 26 at
+// 2.0, 1,587 / 1,633 at 2.2, 1,616 / 1,969 at 2.7, 140 / 1,476 at 160 (82k rows in
+// two colours).  FP32 blocks cross at 1.9; 6x6 ones are longer turns: FP64
+// 2,353 / 2,136 at 1.65 and 27 / 29 at 2.0, FP32 890 / 815 at 1.47 and
+// 2,206 / 2,220 at 1.65.
+int sgs_level_cluster(int32_t n, int bs, bool mixed, const int32_t* fwd_off, int n_fwd, const int32_t* bwd_off,
+                      int n_bwd, int* smem) {
+    if (n <= 0 || (bs != 5 && bs != 6)) return 0;
+    const int C = bs == 5 ? (mixed ? level_cluster<float, 5>(n, smem) : level_cluster<double, 5>(n, smem))
+                          : (mixed ? level_cluster<float, 6>(n, smem) : level_cluster<double, 6>(n, smem));
+    if (C == 0) return 0;
+    const int64_t warps = int64_t(C) * kClusterWarps;
+    int64_t turns = 0;
+    auto count = [&](const int32_t* off, int groups) {
+        for (int g = 0; g < groups; ++g) turns += (off[g + 1] - off[g] + warps - 1) / warps;
+    };
+    count(fwd_off, n_fwd);
+    count(bwd_off, n_bwd);
+    return double(turns) <= (bs == 5 ? 1.9 : 1.65) * (n_fwd + n_bwd) ? C : 0;
 }
 
 template <typename MT>

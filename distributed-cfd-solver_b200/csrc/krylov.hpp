@@ -104,9 +104,11 @@ bool launch_sgs_level_coop(const BsrView& A, const MT* vals, const MT* lu, const
                            int n_bwd, const double* r, double* z, const int* active, cudaStream_t s);
 // The same sweep for a system whose z fits in the shared memory of one
 // cluster: sgs_level_cluster gives the cluster's CTAs and their shared-memory
-// bytes (0: it does not fit, or block sizes other than 5 and 6).  from_zero:
-// z starts from zero (else from the array); z is written once at the end.
-int sgs_level_cluster(int32_t n, int bs, bool mixed, int* smem);
+// bytes (0: it does not fit, its levels are too wide for one cluster, or block
+// sizes other than 5 and 6; offsets on the host).  from_zero: z starts from zero
+// (else from the array); z is written once at the end.  False: not launched.
+int sgs_level_cluster(int32_t n, int bs, bool mixed, const int32_t* fwd_off, int n_fwd, const int32_t* bwd_off,
+                      int n_bwd, int* smem);
 template <typename MT>
 bool launch_sgs_level_cluster(const BsrView& A, const MT* vals, const MT* lu, const int8_t* piv, const int4* fwd_rows,
                               const int32_t* fwd_off, int n_fwd, const int4* bwd_rows, const int32_t* bwd_off,

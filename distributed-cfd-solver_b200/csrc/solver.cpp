@@ -293,8 +293,7 @@ void BsrSystem::set_precision(int precision) {
     }
     precision_ = precision;
     lu_ready_ = false;
-    if (ordering_ == CFDG_SGS_LEVEL)
-        level_cluster_ = sgs_level_cluster(n_, bs_, precision_ == CFDG_PREC_MIXED, &level_smem_);
+    choose_level_sweep();
 }
 
 void BsrSystem::set_values_host(const double* v) {
@@ -488,11 +487,18 @@ void BsrSystem::build_ordering(int ordering) {
         upload_or_throw(fwd_meta_, meta(fr), stream_, "sgs level rows");
         upload_or_throw(bwd_meta_, meta(br), stream_, "sgs level rows");
     }
-    level_cluster_ = ordering == CFDG_SGS_LEVEL ? sgs_level_cluster(n, bs_, precision_ == CFDG_PREC_MIXED, &level_smem_) : 0;
     cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // the host vectors are rebuilt by the next call
     fwd_rows_h_ = std::move(fr);
     bwd_rows_h_ = std::move(br);
     ordering_ = ordering;
+    choose_level_sweep();
+}
+
+void BsrSystem::choose_level_sweep() {
+    level_cluster_ = 0;
+    if (ordering_ == CFDG_SGS_LEVEL)
+        level_cluster_ = sgs_level_cluster(n_, bs_, precision_ == CFDG_PREC_MIXED, fwd_off_.data(), groups_fwd(),
+                                           bwd_off_.data(), groups_bwd(), &level_smem_);
 }
 
 // Blocks and unique-touch bytes of every pass of the ordering (profiling).
@@ -797,10 +803,11 @@ void BsrSystem::sgs_apply_t(const MT* vals, const MT* lu, const double* r, doubl
     // sweep; with two colours every neighbour of the second colour is of the
     // first colour, and the split sweep never reads them, so no clearing is
     // needed then.
-    if ((!color && level_cluster_ == 0) || (color && nf > 2 && !split_)) {
+    auto clear = [&] {
         ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 0, 8.0 * n_ * bs_);
         cuda_check(cudaMemsetAsync(z, 0, sizeof(double) * static_cast<std::size_t>(n_) * bs_, stream_), "memset");
-    }
+    };
+    if ((!color && level_cluster_ == 0) || (color && nf > 2 && !split_)) clear();
     for (int sw = 0; sw < sweeps_; ++sw) {
         const bool split = split_ && sw == 0;
         if (!color && (level_cluster_ > 0 || level_coop_)) {
@@ -810,13 +817,15 @@ void BsrSystem::sgs_apply_t(const MT* vals, const MT* lu, const double* r, doubl
             for (int g = 0; g < nbk; ++g) bytes += bwd_bytes_[0][g] + bwd_blocks_[0][g] * block_bytes();
             ProfScope ps(prof_, CFDG_KCAT_SGS, stream_, 1, bytes);
             if (level_cluster_ > 0) {
-                if (!launch_sgs_level_cluster<MT>(A, vals, lu, piv_.p, fwd_meta_.p, fwd_off_d_.p, nf, bwd_meta_.p,
-                                                  bwd_off_d_.p, nbk, r, z, sw == 0, level_cluster_, level_smem_, active,
-                                                  stream_))
-                    cuda_check(cudaGetLastError(), "level sweep launch");
-                continue;
+                if (launch_sgs_level_cluster<MT>(A, vals, lu, piv_.p, fwd_meta_.p, fwd_off_d_.p, nf, bwd_meta_.p,
+                                                 bwd_off_d_.p, nbk, r, z, sw == 0, level_cluster_, level_smem_, active,
+                                                 stream_))
+                    continue;
+                cudaGetLastError();
+                level_cluster_ = 0;  // the grid-wide sweep takes over
+                if (sw == 0) clear();
             }
-            if (fwd_meta_.p &&
+            if (fwd_meta_.p && level_coop_ &&
                 launch_sgs_level_coop<MT>(A, vals, lu, piv_.p, fwd_meta_.p, fwd_off_d_.p, nf, bwd_meta_.p,
                                           bwd_off_d_.p, nbk, r, z, active, stream_))
                 continue;

@@ -196,6 +196,7 @@ public:
 
 private:
     void build_ordering(int ordering);
+    void choose_level_sweep();
     void count_pass_bytes();
     bool bytes_counted_ = false;
     template <typename F>

@@ -1,12 +1,15 @@
-"""The level-scheduled sweep in one thread-block cluster against the
-sequential sweep in numpy: one row, rows with more off-diagonal blocks than a
-warp fetches ahead, one and two sweeps, both precisions, and sizes around the
-largest whose z fits in a 16-CTA cluster (5 x 5 blocks: 16 x 204,800 / 40 =
-81,920 rows; one more row takes the grid-wide sweep).
+"""The level-scheduled sweep, in one thread-block cluster or over the grid,
+against the sequential sweep in numpy: one row, rows with more off-diagonal
+blocks than a warp fetches ahead, one and two sweeps, both precisions, sizes
+around the largest whose z fits in a 16-CTA cluster (5 x 5 blocks: 16 x 204,800 /
+40 = 81,920 rows; one more row takes the grid-wide sweep), and levels of up to
+256 rows (the cluster's), a little more and half of the matrix (the grid's).
 
 1e-12: FP64 substitutions of well-conditioned blocks (unit roundoff times the
 rows a value passes through); the FP32 matrix is compared with the numpy sweep
 on the rounded values and FP32-rounded factors, 2e-6."""
+import time
+
 import numpy as np
 import pytest
 
@@ -62,7 +65,7 @@ def test_matches_sequential_sweep(cb, n, bs, degree, mixed, sweeps):
 
 @pytest.mark.parametrize("n", [81918, 81920, 81922])
 def test_largest_cluster_sizes(cb, n):
-    """Coupled pairs of rows: two levels, any size, a closed form."""
+    """Coupled pairs of rows: two wide levels, any size, a closed form."""
     bs, rng = 5, np.random.default_rng(5)
     row_ptr = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
     first = np.arange(0, n, 2)
@@ -85,3 +88,56 @@ def test_largest_cluster_sizes(cb, n):
     z0 = solve(d0, r[0::2] - np.einsum("kij,kj->ki", u, z1))
     assert rel_err(z[1::2], z1) < 1e-12
     assert rel_err(z[0::2], z0) < 1e-12
+
+
+@pytest.mark.parametrize("n,width", [(81918, 256), (81920, 256), (81922, 256), (10241, 255), (10300, 480), (10300, 520)])
+def test_chains(cb, n, width):
+    """`width` chains of rows side by side: level k is rows k * width on, solved
+    for all chains at once in numpy."""
+    bs, rng = 5, np.random.default_rng(6)
+    i = np.arange(n)
+    cols = np.stack([i - width, i, i + width], axis=1)
+    have = (cols >= 0) & (cols < n)
+    row_ptr = np.concatenate([[0], np.cumsum(have.sum(axis=1))]).astype(np.int32)
+    vals = 0.3 * rng.standard_normal((n, 3, bs, bs))
+    vals[:, 1] += 4.0 * np.eye(bs)
+    r = rng.standard_normal((n, bs))
+    A = cb.Bsr(row_ptr, cols[have].astype(np.int32), bs)
+    A.set_values(vals[have])
+    A.sgs_setup(cb.SGS_LEVEL, 1)
+    z = np.zeros((n, bs))
+    for side in (0, 2):
+        for k in (range(0, n, width) if side == 0 else reversed(range(0, n, width))):
+            q = slice(k, min(k + width, n))
+            s = r[q].copy()
+            for c in (0, 2):
+                m = have[q, c]
+                s[m] -= np.einsum("kij,kj->ki", vals[q, c][m], z[cols[q, c][m]])
+            z[q] = np.linalg.solve(vals[q, 1], s[:, :, None])[:, :, 0]
+    assert rel_err(A.sgs_apply(r.ravel()).reshape(n, bs), z) < 1e-12
+
+
+def test_wide_levels_take_the_whole_gpu(cb):
+    """Two levels of 20,000 rows, 61 us a sweep over the grid: 5.9 times the
+    multicolour sweep of the same rows.  One cluster takes 566 us, 54 times; the
+    bound of 18 lies between."""
+    n, bs, sweeps = 40000, 5, 40
+    row_ptr = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    half = np.arange(n // 2)
+    cols = np.concatenate([np.stack([half, half + n // 2], axis=1)] * 2).astype(np.int32).ravel()
+    vals = np.tile(0.1 * np.ones((bs, bs)), (2 * n, 1, 1))
+    vals[np.repeat(np.arange(n), 2) == cols] += 4.0 * np.eye(bs)
+    r = np.random.default_rng(7).standard_normal(n * bs)
+    times = {}
+    for ordering in (cb.SGS_COLOR, cb.SGS_LEVEL):
+        A = cb.Bsr(row_ptr, cols, bs)
+        A.set_values(vals)
+        took = {}
+        for count in (1, sweeps):  # the difference leaves the copies out
+            A.sgs_setup(ordering, count)
+            for _ in range(6):
+                t = time.perf_counter()
+                A.sgs_apply(r)
+                took.setdefault(count, []).append(time.perf_counter() - t)
+        times[ordering] = min(took[sweeps]) - min(took[1])
+    assert times[cb.SGS_LEVEL] < 18.0 * times[cb.SGS_COLOR]
