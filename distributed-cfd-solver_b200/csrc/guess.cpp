@@ -135,31 +135,21 @@ void Mlp::queue_grad(const uint16_t* X, const float* T, int64_t rows, bool adam,
     if (adam) ++step_;
     const double inv = 1.0 / (double(rows) * nvars_);
     launch_mlp_adam(params_, m_, v_, w_, partials_, parts, inv, lr, 0.9f, 0.999f, 1e-8f, std::max(step_, 1), adam,
-                    grad_, loss_dev, s);
+                    grad_, loss_dev, err_, s);
     launches_ += 2;
     cuda_check(cudaGetLastError(), "mlp train launch");
 }
 
-float Mlp::read_loss(cudaStream_t s) {
+float Mlp::gradient(const uint16_t* X, const float* T, int64_t rows, float* grad_host, cudaStream_t s) {
+    queue_grad(X, T, rows, false, 0.0f, loss_, s);
     float loss = 0.0f;
     cuda_check(cudaMemcpyAsync(&loss, loss_, sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
     check_err(s);
-    return loss;
-}
-
-float Mlp::gradient(const uint16_t* X, const float* T, int64_t rows, float* grad_host, cudaStream_t s) {
-    queue_grad(X, T, rows, false, 0.0f, loss_, s);
-    const float loss = read_loss(s);
     if (grad_host) {
         cuda_check(cudaMemcpyAsync(grad_host, grad_, kMlpParams * sizeof(float), cudaMemcpyDeviceToHost, s), "D2H");
         cuda_check(cudaStreamSynchronize(s), "sync");
     }
     return loss;
-}
-
-float Mlp::adam_step(const uint16_t* X, const float* T, int64_t rows, float lr, cudaStream_t s) {
-    queue_grad(X, T, rows, true, lr, loss_, s);
-    return read_loss(s);
 }
 
 float Mlp::train(const Dataset& ds, int epochs, int batch, float lr, uint64_t seed, cudaStream_t s) {
@@ -181,17 +171,26 @@ float Mlp::train(const Dataset& ds, int epochs, int batch, float lr, uint64_t se
         losses_cap_ = nb;
     }
     std::vector<float> host(static_cast<std::size_t>(nb));
+    const std::size_t bytes = sizeof(float) * static_cast<std::size_t>(nb);
     float last = 0.0f;
     for (int e = 0; e < epochs; ++e) {
         std::shuffle(order.begin(), order.end(), g);
+        cuda_check(cudaMemsetAsync(losses_, 0xFF, bytes, s), "memset");  // no batch applied yet
         for (int64_t k : order) {
             const int64_t r0 = k * batch, rows = std::min<int64_t>(batch, n - r0);
             queue_grad(ds.X() + r0 * kMlpIn, ds.T() + r0 * kMlpOut, rows, true, lr, losses_ + k, s);
         }
-        cuda_check(cudaMemcpyAsync(host.data(), losses_, sizeof(float) * static_cast<std::size_t>(nb),
-                                   cudaMemcpyDeviceToHost, s),
-                   "D2H");
-        check_err(s);
+        cuda_check(cudaMemcpyAsync(host.data(), losses_, bytes, cudaMemcpyDeviceToHost, s), "D2H");
+        try {
+            check_err(s);
+        } catch (...) {  // the network stands at the last good batch
+            for (float loss : host) {
+                uint32_t bits;
+                std::memcpy(&bits, &loss, sizeof(bits));
+                if (bits == 0xFFFFFFFFu) --step_;
+            }
+            throw;
+        }
         double acc = 0.0;
         for (int64_t k : order)
             acc += double(host[static_cast<std::size_t>(k)]) * double(std::min<int64_t>(batch, n - k * batch));

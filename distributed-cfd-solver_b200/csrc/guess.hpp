@@ -40,8 +40,6 @@ public:
     // loss (mean squared error over rows x nvars) and, when grad_host is
     // set, its gradient; no update
     float gradient(const uint16_t* X, const float* T, int64_t rows, float* grad_host, cudaStream_t s);
-    // one Adam step on the batch; returns the batch loss before the step
-    float adam_step(const uint16_t* X, const float* T, int64_t rows, float lr, cudaStream_t s);
     // epochs over the dataset in shuffled contiguous batches; mean loss of the last epoch
     float train(const Dataset& ds, int epochs, int batch, float lr, uint64_t seed, cudaStream_t s);
     int64_t launches() const { return launches_; }
@@ -64,7 +62,6 @@ private:
     // gradient and optional Adam step of a batch; its loss goes to *loss_dev
     void queue_grad(const uint16_t* X, const float* T, int64_t rows, bool adam, float lr, float* loss_dev,
                     cudaStream_t s);
-    float read_loss(cudaStream_t s);
     void check_err(cudaStream_t s);
 };
 

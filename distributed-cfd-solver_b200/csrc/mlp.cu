@@ -539,14 +539,17 @@ __global__ void __launch_bounds__(128, 1) k_mlp_grad(MlpDev net, const uint16_t*
 // One Adam step.  kAdamSlices threads share a parameter: slice q adds the
 // CTAs q, q + kAdamSlices, ... in order, the slices' sums follow one another.
 // The updated weights leave in bf16 as well, in both orientations the products
-// read.  Bound by the latency of the partials' loads (a few MB in L2).
+// read.  Bound by the latency of the partials' loads (a few MB in L2).  Once
+// *err is set (a wait of this batch or an earlier one gave up, its partials are
+// not whole) nothing is written any more.
 constexpr int kAdamParams = 32, kAdamSlices = 8;
 
 __global__ void __launch_bounds__(kAdamParams * kAdamSlices)
     k_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials,
                int nparts, double inv_count, float lr, float b1, float b2, float eps, float c1, float c2, bool adam,
-               float* grad_out, float* loss_out) {
+               float* grad_out, float* loss_out, const int* err) {
     pdl_enter();
+    const int failed = *err;  // on its way while the partials load
     __shared__ double sh[kAdamSlices][kAdamParams];
     const int local = threadIdx.x % kAdamParams, slice = threadIdx.x / kAdamParams;
     const int p = blockIdx.x * kAdamParams + local;
@@ -557,7 +560,7 @@ __global__ void __launch_bounds__(kAdamParams * kAdamSlices)
     }
     sh[slice][local] = part;
     __syncthreads();
-    if (slice != 0 || p > kMlpParams) return;
+    if (slice != 0 || p > kMlpParams || failed) return;
     double acc = sh[0][local];
 #pragma unroll
     for (int q = 1; q < kAdamSlices; ++q) acc += sh[q][local];
@@ -616,10 +619,10 @@ int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target
 
 void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials, int nparts,
                      double inv_count, float lr, float beta1, float beta2, float eps, int step, bool adam,
-                     float* grad_out, float* loss_out, cudaStream_t s) {
+                     float* grad_out, float* loss_out, const int* err, cudaStream_t s) {
     const float c1 = 1.0f - powf(beta1, float(step)), c2 = 1.0f - powf(beta2, float(step));
     launch_after(k_mlp_adam, (kMlpParams + kAdamParams) / kAdamParams, kAdamParams * kAdamSlices, 0, s, params, m, v, w,
-                 partials, nparts, inv_count, lr, beta1, beta2, eps, c1, c2, adam, grad_out, loss_out);
+                 partials, nparts, inv_count, lr, beta1, beta2, eps, c1, c2, adam, grad_out, loss_out, err);
 }
 
 }  // namespace cfdg

@@ -58,9 +58,10 @@ int launch_mlp_grad(const MlpDev& net, const uint16_t* feat, const float* target
 
 // Sums the CTA partials in fixed order, scales by 1/(rows * nout), and
 // applies one Adam step, refreshing the bf16 copies `w` (or only writes the
-// gradient when adam == false).
+// gradient when adam == false).  err: the error flag of launch_mlp_grad; once it
+// is set, nothing is written.
 void launch_mlp_adam(float* params, float* m, float* v, uint16_t* w, const float* partials, int nparts,
                      double inv_count, float lr, float beta1, float beta2, float eps, int step, bool adam,
-                     float* grad_out, float* loss_out, cudaStream_t s);
+                     float* grad_out, float* loss_out, const int* err, cudaStream_t s);
 
 }  // namespace cfdg

@@ -9,6 +9,11 @@ with the median entry below 1e-4 (a hidden activation that lands on the
 other side of a bf16 rounding boundary moves one output by ~2^-9 of that
 unit's contribution); gradient 2e-2 in norm; loss 1e-5.
 """
+import ctypes as C
+import os
+import subprocess
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -234,3 +239,36 @@ def test_host_samples_are_on_the_device_before_the_kernel(cb):
     for _ in range(60):
         loss, h = net.gradient(X, T)
         assert loss == first and np.array_equal(g, h)
+
+
+def test_failed_batch_leaves_the_network(tmp_path):
+    """After a batch whose kernel reported an error, no batch of the epoch changes
+    the parameters or counts as a step, and the call reports it (the flag is set
+    from the host)."""
+    root = Path(__file__).resolve().parents[1]
+    so = tmp_path / "failed_batch.so"
+    subprocess.run([os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc"), "-gencode", "arch=compute_100a,code=sm_100a",
+                    "-std=c++17", "-shared", "-Xcompiler", "-fPIC", f"-I{root / 'include'}",
+                    f"-I{root / 'distributed-cfd-solver_b200' / 'csrc'}", "-o", str(so),
+                    str(root / "tests" / "mlp_failed_batch.cu")], check=True, capture_output=True)
+    lib = C.CDLL(str(so))
+    rows, batch, rng = 1000, 256, np.random.default_rng(5)
+    x = np.zeros((rows, M.IN), dtype=np.uint16)
+    x[:, :] = rng.integers(0x3E80, 0x3F80, x.shape)  # bf16 values of 0.25 to 1
+    t = rng.standard_normal((rows, M.OUT)).astype(np.float32)
+
+    def train(rows, fail):
+        p = np.zeros(M.N_PARAMS, dtype=np.float32)
+        steps = lib.train(rows, batch, fail, x.ctypes.data_as(C.c_void_p), t.ctypes.data_as(C.c_void_p),
+                          p.ctypes.data_as(C.c_void_p))
+        return steps, p
+
+    steps, trained = train(rows, 0)
+    assert steps == 4
+    steps, kept = train(rows, 1)
+    assert steps == 0
+    assert np.isfinite(kept).all() and np.abs(trained - kept).max() > 1e-3
+    assert np.array_equal(kept, train(rows, 1)[1])
+    # the parameters are the initial ones: one good batch from them gives the first Adam step, lr wide at most
+    steps, one = train(batch, 0)
+    assert steps == 1 and 0.0 < np.abs(one - kept).max() <= 1.001e-2
