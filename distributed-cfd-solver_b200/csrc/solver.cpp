@@ -285,6 +285,8 @@ void BsrSystem::set_precision(int precision) {
     if (precision == CFDG_PREC_MIXED) {
         vals64_.release();
         lu64_.release();
+        mid_.release();
+        w_.release();
         alloc_or_throw(vals32_, nv, "values");
     } else {
         vals32_.release();
@@ -449,18 +451,9 @@ void BsrSystem::build_ordering(int ordering) {
     // is of the other colour.
     const int ncolor = static_cast<int>(fwd_off_.size()) - 1;
     reducible_ = reduce && ordering == CFDG_SGS_COLOR && ncolor >= 2 && (split_ || ncolor == 2);
-    if (reducible_) {
-        std::vector<int32_t> mid(n);
-        for (int32_t i = 0; i < n; ++i) {
-            int32_t k = row_ptr_h_[i];
-            while (k < diag_h_[i] && fwd_key[cols_h_[k]] == 0) ++k;
-            mid[i] = k;
-        }
-        upload_or_throw(mid_, mid, stream_, "sgs row splits");
-        cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // mid dies here
-        if (!w_.p) alloc_or_throw(w_, static_cast<std::size_t>(n) * bs_, "krylov");
-    }
     release_red_graphs();
+    mid_.release();
+    w_.release();
     // the passes' byte counts are formed when a profiler asks for them
     bytes_counted_ = false;
     for (int m = 0; m < 3; ++m) {
@@ -499,6 +492,25 @@ void BsrSystem::choose_level_sweep() {
     if (ordering_ == CFDG_SGS_LEVEL)
         level_cluster_ = sgs_level_cluster(n_, bs_, precision_ == CFDG_PREC_MIXED, fwd_off_.data(), groups_fwd(),
                                            bwd_off_.data(), groups_bwd(), &level_smem_);
+}
+
+// The reduced solve's own arrays, after those that every solve needs; where they
+// do not fit, the solve takes the full form.
+void BsrSystem::red_alloc() {
+    std::vector<char> first(n_, 0);
+    for (int32_t q = 0; q < fwd_off_[1]; ++q) first[fwd_rows_h_[q]] = 1;
+    std::vector<int32_t> mid(n_);
+    for (int32_t i = 0; i < n_; ++i) {
+        int32_t k = row_ptr_h_[i];
+        while (k < diag_h_[i] && first[cols_h_[k]]) ++k;
+        mid[i] = k;
+    }
+    if (!mid_.upload(mid, stream_) || !w_.alloc(static_cast<std::size_t>(n_) * bs_)) {
+        cudaGetLastError();
+        reducible_ = false;
+    }
+    cuda_check(cudaStreamSynchronize(stream_), "setup sync");  // mid dies here
+    if (!reducible_) mid_.release();
 }
 
 // Blocks and unique-touch bytes of every pass of the ordering (profiling).
@@ -621,6 +633,7 @@ void BsrSystem::sgs_setup(int ordering, int sweeps, bool check) {
         ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + bs_ + 4.0));
         launch_lu_setup<double>(view(), vals64_.p, lu64_.p, piv_.p, err_.p, color, stream_);
     }
+    if (reducible() && !w_.p) red_alloc();
     if (reducible()) {
         ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 1, double(n_) * (b2 * 16.0 + 4.0));
         launch_red_check(red_view(), vals64_.p, lu64_.p, err_.p + 1, stream_);

@@ -198,6 +198,7 @@ private:
     void build_ordering(int ordering);
     void choose_level_sweep();
     void count_pass_bytes();
+    void red_alloc();
     bool bytes_counted_ = false;
     template <typename F>
     bool device_loop_ready(int precond, double* x, const double* b, F&& iteration);

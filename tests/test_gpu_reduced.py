@@ -101,3 +101,36 @@ def test_long_solves(cb, order, cond):
         x, info = A.bicgstab(b, rel_tol=1e-10, max_it=500)
         assert info.status == cb.KRYLOV_CONVERGED and info.iterations > 32
         assert np.linalg.norm(b - M @ x) <= 1.01e-10 * np.linalg.norm(b)
+
+
+def test_set_up_at_the_memory_limit(cb):
+    """Memory for the factors (115 MB, pivots, row lists) and 8 MB more, but not for
+    the reduced solve's 21 MB of vectors: the solve takes the full form."""
+    torch = pytest.importorskip("torch")
+    n, bs = 400000, 6
+    half = np.arange(n // 2)
+    row_ptr = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    cols = np.concatenate([np.stack([half, half + n // 2], axis=1)] * 2).astype(np.int32).ravel()
+    vals = np.tile(0.1 * np.ones((bs, bs)), (2 * n, 1, 1))
+    vals[np.repeat(np.arange(n), 2) == cols] += 4.0 * np.eye(bs)
+    b = np.random.default_rng(3).standard_normal(n * bs)
+
+    def solve(A):
+        A.sgs_setup(cb.SGS_COLOR, 1)
+        return A.bicgstab(b, rel_tol=1e-10, max_it=20)
+
+    first = cb.Bsr(row_ptr, cols, bs)  # loads the kernels
+    first.set_values(vals)
+    x, _ = solve(first)
+    first.close()
+    A = cb.Bsr(row_ptr, cols, bs)
+    A.set_values(vals)
+    room = n * (bs * bs * 8 + bs + 4 * 4) + (8 << 20)
+    torch.cuda.synchronize()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda")
+    A.sgs_setup(cb.SGS_COLOR, 1)
+    del hold
+    torch.cuda.empty_cache()
+    y, info = A.bicgstab(b, rel_tol=1e-10, max_it=20)
+    assert info.status == cb.KRYLOV_CONVERGED
+    assert rel_err(y, x) < 1e-9
