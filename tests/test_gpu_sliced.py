@@ -15,10 +15,23 @@ CASES = {  # odd sizes whose matrix is a little over twice L2
 }
 
 
+def _slices(s):
+    """Whether a step keeps a sliced copy: its set-up profiles the factorisation and
+    the copies, else the factorisation alone."""
+    s.profile(True)
+    s.newton_step(5.0)
+    launches = s.profile_read()["lu"]["launches"]
+    s.profile(False)
+    assert launches in (1, 2)
+    return launches == 2
+
+
 def _steps(cb, case, mesh, loop, state):
     case.cfg.krylov_loop = loop
     out = []
     with cb.Solver(mesh, case.cfg, case.bcs) as s:
+        s.set_state(state)
+        assert _slices(s) == (loop == cb.KRYLOV_DEVICE_LOOP)
         s.set_state(state)
         for _ in range(2):
             r = s.newton_step(5.0)
@@ -33,6 +46,7 @@ def test_slices_are_the_rows(cb, name, sweeps):
     case = getattr(cb.cases, make)(mixed=mixed)
     case.spec.nx, case.spec.ny, case.spec.nz = size
     case.cfg.sgs_sweeps = sweeps
+    case.cfg.pre_freeze = cb.PREFREEZE_CONFIGURED  # FP32 from the first step on
     case.cfg.lin_rel_tol, case.cfg.lin_abs_tol, case.cfg.lin_max_iterations = 1e-30, 1e-300, 6
     mesh = cb.HostMesh(case.spec)
     state = cb.cases.perturbed_state(case, mesh.n_cells)
