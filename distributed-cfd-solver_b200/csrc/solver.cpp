@@ -744,17 +744,28 @@ void BsrSystem::build_sell() {
     sell_ordering_ = ordering_;
 }
 
-// The sliced copy of the current values and diagonal inverses.
+// The sliced copy of the current values and diagonal inverses.  Where memory is
+// short the passes read the matrix itself, and every 32nd set-up looks again (a
+// look, cudaMemGetInfo, waits for the device).
 void BsrSystem::fill_sell() {
+    constexpr int kLookAgain = 32;
     sell_on_ = false;
     if (!sell_wanted()) return;
+    if (sell_wait_ > 0) {
+        --sell_wait_;
+        return;
+    }
     const int64_t b2 = int64_t(bs_) * bs_;
     try {
         if (!sell32_.p && !sell64_.p) {  // a second copy of the matrix only where memory is ample
             std::size_t room = 0, total = 0;
             cuda_check(cudaMemGetInfo(&room, &total), "cudaMemGetInfo");
-            if (!sell_ready(bs_, precision_ == CFDG_PREC_MIXED) || 8.0 * double(nnzb_) * block_bytes() > double(room)) {
+            if (!sell_ready(bs_, precision_ == CFDG_PREC_MIXED)) {
                 sell_failed_ = true;
+                return;
+            }
+            if (8.0 * double(nnzb_) * block_bytes() > double(room)) {
+                sell_wait_ = kLookAgain - 1;
                 return;
             }
         }
@@ -770,9 +781,9 @@ void BsrSystem::fill_sell() {
         }
     } catch (const Failure& f) {
         if (f.status != CFDG_ERR_NOMEM) throw;
-        cudaGetLastError();  // no room for a second copy: the passes read the matrix itself
+        cudaGetLastError();
         release_sell();
-        sell_failed_ = true;
+        sell_wait_ = kLookAgain - 1;
         return;
     }
     ProfScope ps(prof_, CFDG_KCAT_LU, stream_, 2, 2.0 * (double(nnzb_) + n_) * block_bytes());
@@ -789,7 +800,8 @@ void BsrSystem::fill_sell() {
 }
 
 void BsrSystem::release_sell() {
-    sell_on_ = false;
+    sell_on_ = sell_failed_ = false;
+    sell_wait_ = 0;
     sell64_.release();
     sellinv64_.release();
     sell32_.release();

@@ -213,7 +213,8 @@ private:
     void fill_sell();
     void release_sell();
     void sell_pass(int kind, int c0, int c1, const double* r, double* z, double* y, const int* active);
-    bool sell_on_ = false, sell_failed_ = false;
+    bool sell_on_ = false, sell_failed_ = false;  // failed: the device cannot run the passes
+    int sell_wait_ = 0;                           // set-ups until memory is looked at again
     int sell_ordering_ = -1;
     std::vector<int32_t> sell_first_;  // first slice of each colour
     int64_t sell_columns_ = 0, sell_diag0_ = 0;

@@ -53,3 +53,23 @@ def test_slices_are_the_rows(cb, name, sweeps):
     a, b = (_steps(cb, case, mesh, loop, state) for loop in (cb.KRYLOV_DEVICE_LOOP, cb.KRYLOV_HOST_LOOP))
     assert a[0] == b[0]
     assert np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2])
+
+
+def test_slices_come_when_memory_does(cb):
+    """Less memory than eight times the copy at the first steps: the rows are used,
+    and the slices once it is free again."""
+    torch = pytest.importorskip("torch")
+    make, size, mixed = CASES["plate_fp64"]
+    case = getattr(cb.cases, make)(mixed=mixed)
+    case.spec.nx, case.spec.ny, case.spec.nz = size
+    case.cfg.lin_max_iterations = 2
+    mesh = cb.HostMesh(case.spec)
+    with cb.Solver(mesh, case.cfg, case.bcs) as s:
+        s.set_state(cb.cases.perturbed_state(case, mesh.n_cells))
+        hold = torch.empty(torch.cuda.mem_get_info()[0] - (1500 << 20), dtype=torch.uint8, device="cuda")
+        assert not _slices(s)
+        del hold
+        torch.cuda.empty_cache()
+        for _ in range(32):
+            s.newton_step(5.0)
+        assert _slices(s)
