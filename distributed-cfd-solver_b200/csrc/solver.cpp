@@ -1094,7 +1094,7 @@ void BsrSystem::red_end() {
 // error on the way leaves the host loop in charge.
 bool BsrSystem::red_graph_ready(Start start) {
     if (red_exec_[start]) return true;
-    if (loop_failed_) return false;
+    if (red_failed_) return false;
     const int64_t launches0 = prof_->launches;
     cudaGraph_t g = nullptr;
     bool capturing = false;
@@ -1145,7 +1145,7 @@ bool BsrSystem::red_graph_ready(Start start) {
         }
         cudaGetLastError();
         red_exec_[start] = nullptr;
-        loop_failed_ = true;
+        red_failed_ = true;
     }
     red_fixed_launches_[start] = prof_->launches - launches0 - red_body_launches_;
     prof_->launches = launches0;
@@ -1442,8 +1442,8 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
     const double bnorm = std::sqrt(hh[2 * m + 2]);
     double beta = bnorm;
     int guess_state = 0;
-    // x holds x0; with the matrix-free product and no guess the caller has
-    // zeroed it, and r0 = b needs no residual evaluation
+    // x holds x0; with the matrix-free product and no guess it is cleared below,
+    // whatever it holds, and r0 = b needs no residual evaluation
     bool zero_start = product_ && !guess;
     if (!zero_start) {
         apply_A(x, vec(0));

@@ -289,6 +289,7 @@ private:
     // caller's x and b are read through the device scalars)
     cudaGraphExec_t red_exec_[3] = {nullptr, nullptr, nullptr};
     int64_t red_fixed_launches_[3] = {0, 0, 0}, red_body_launches_ = 0;
+    bool red_failed_ = false;  // a capture failed: the host loop runs the reduced solve
     KrylovScalars* ks_init_ = nullptr;  // pinned: the scalars a solve starts from
     // rows [fwd_off_[1], n) of a colour-ordered matrix: block count and
     // distinct columns (the SpMV left after the fused colour-0 product)
