@@ -1943,9 +1943,13 @@ void Solver::setup_matrix(const HostMesh& hm, const Csr& c2c) {
     // the wall-stretched viscous systems an unconverged solve amplifies
     // rounding up to 1e13 times (two solves whose input differs by one unit in
     // the last place end 1e-3 apart on the Spalart-Allmaras plate, 30
-    // iterations): there the full solve stays.  Inviscid FP64 solves agree to
-    // 1e-12, and are 1.2x faster (4,096-cell ramp, ten steady
-    // iterations: 2.91 -> 2.41 ms).
+    // iterations): there the full solve stays.  Inviscid FP64 steps amplify less:
+    // over 60 drawn ones (ramps and tetrahedral bumps of 40 to 22,000 cells, 1 to 5
+    // steps, steady and dual time, 5 to 40 iterations) the update moves by 0.5
+    // times what one unit in the last place of the state moves the full form's,
+    // at most 5.9 times; up to the benchmark flows' CFL of 100 the state stays within
+    // 1e-10, at CFL 1,600 both move by up to 1e-5.  They are 1.2x faster
+    // (4,096-cell ramp, ten steady iterations: 2.91 -> 2.41 ms).
     sys_->reduce = cfg_.viscous == 0;
     auto pos = [&](int32_t row, int32_t col) -> int32_t {
         const auto b = cols.begin() + row_ptr[row], e = cols.begin() + row_ptr[row + 1];
