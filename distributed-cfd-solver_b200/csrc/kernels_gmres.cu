@@ -1,7 +1,7 @@
 // Restarted GMRES building blocks (right-preconditioned, classical
 // Gram-Schmidt with one reorthogonalisation pass).  The Krylov basis is one
 // array of (restart + 1) vectors of `len` doubles; the projections go
-// through fused multi-dot products (up to kGmChunk basis vectors against w
+// through fused multi-dot products (up to gm_chunk(len) basis vectors against w
 // per launch, w read once per launch) and one fused update
 // w -= sum_k h_k V_k.  Reductions are per block in a fixed order, then a
 // finaliser per coefficient over the blocks in block order: the grid depends
@@ -14,7 +14,7 @@ namespace {
 
 constexpr int kGmThreads = 256;
 constexpr int64_t kGmGridCap = 148 * 8;
-constexpr int kGmChunk = 24;
+constexpr int kGmChunk = 24, kGmLongChunk = 8;
 
 inline unsigned gm_grid(int64_t len) {
     const int64_t g = grid_for(len, kGmThreads);
@@ -22,12 +22,16 @@ inline unsigned gm_grid(int64_t len) {
 }
 
 // partials[b * C + k] = sum over block b's entries of V_{k0+k} . w, k < kn
-// (kn <= C).  V = w with kn = 1 gives |w|^2.  A vector of a million entries is
-// a few entries a thread, so a launch is latency: all C basis entries load at
-// once, and C follows the number of vectors (8, 16 or 24) so that a basis of
-// 24 is one launch instead of three.  With this, the update's norm in the same
-// pass and the host reading a column while the next product runs, a
-// Jacobian-free step of the 131k-cell plate takes 7.08 ms instead of 7.20.
+// (kn <= C).  V = w with kn = 1 gives |w|^2.  While a thread has one entry (up to
+// 303,104), a launch is latency: all C basis entries load at once, and C follows
+// the number of vectors (8, 16 or 24) so that a basis of 24 is one launch instead
+// of three.  Longer vectors are bound by memory, where the fewer blocks that 24
+// sums leave room for cost more than reading w again: they go by eight.  The 60
+// launches' products of a 30-vector cycle, us, 24 / 8 a launch: 725 / 902 at 80k
+// entries, 1,423 / 1,479 at 240k, 2,413 / 2,152 at 655k, 9,391 / 7,173 at 4.1M.  With
+// the update's norm in the same pass and the host reading a column while the next
+// product runs, a Jacobian-free step of the 131k-cell plate takes 7.08 ms instead
+// of 7.20.
 template <int C>
 __global__ void __launch_bounds__(kGmThreads) k_gm_dots(int64_t len, const double* V, int64_t ld, int k0,
                                                         int kn, const double* w,
@@ -111,13 +115,14 @@ __global__ void __launch_bounds__(kGmThreads) k_gm_axpy(int64_t len, double a, c
 }  // namespace
 
 int gm_partial_blocks(int64_t len) { return static_cast<int>(gm_grid(len)); }
-int gm_chunk() { return kGmChunk; }
+int gm_chunk(int64_t len) { return len <= kGmGridCap * kGmThreads ? kGmChunk : kGmLongChunk; }
 
 void launch_gm_dots(int64_t len, const double* V, int64_t ld, int k0, int kn, const double* w, double* partials,
                     double* h, cudaStream_t s) {
     const unsigned gr = gm_grid(len);
-    for (int c = 0; c < kn; c += kGmChunk) {
-        const int m = kn - c < kGmChunk ? kn - c : kGmChunk;
+    const int chunk = gm_chunk(len);
+    for (int c = 0; c < kn; c += chunk) {
+        const int m = kn - c < chunk ? kn - c : chunk;
         const int stride = m == 1 ? 1 : m <= 8 ? 8 : m <= 16 ? 16 : 24;
         if (m == 1) launch_after(k_gm_dots<1>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);
         else if (m <= 8) launch_after(k_gm_dots<8>, gr, kGmThreads, 0, s, len, V, ld, k0 + c, m, w, partials);

@@ -1367,7 +1367,7 @@ void BsrSystem::gm_alloc(int restart) {
     gm_V_.release();
     alloc_or_throw(gm_V_, N * (restart + 1), "GMRES basis");
     alloc_or_throw(gm_z_, N, "GMRES vector");
-    alloc_or_throw(gm_part_, static_cast<std::size_t>(gm_partial_blocks(int64_t(N))) * gm_chunk() + 8, "GMRES partials");
+    alloc_or_throw(gm_part_, static_cast<std::size_t>(gm_partial_blocks(int64_t(N))) * gm_chunk(int64_t(N)) + 8, "GMRES partials");
     alloc_or_throw(gm_h_, 3 * static_cast<std::size_t>(restart + 1) + 8, "GMRES coefficients");
     cuda_check(cudaMemsetAsync(gm_h_.p, 0, gm_h_.count * sizeof(double), stream_), "memset");
     if (!gm_read_) cuda_check(cudaEventCreateWithFlags(&gm_read_, cudaEventDisableTiming), "cudaEventCreate");
@@ -1416,7 +1416,7 @@ cfdg_krylov_result BsrSystem::gmres(int precond, double rel_tol, double abs_tol,
             cuda_check(cudaMemcpyAsync(z, r, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream_), "D2D");
         }
     };
-    const int chunk = gm_chunk();
+    const int chunk = gm_chunk(N);
     auto dots = [&](int kn, const double* w, double* h) {
         ProfScope ps(prof_, CFDG_KCAT_KRYLOV, stream_, 2 * ((kn + chunk - 1) / chunk),
                      8.0 * N * (kn + (kn + chunk - 1) / chunk));
