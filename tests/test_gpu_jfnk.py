@@ -135,3 +135,30 @@ def test_jacobian_free_options_are_checked(cb, field, value):
     mesh = cb.HostMesh(case.spec)
     with pytest.raises(cb.CfdgError):
         cb.Solver(mesh, case.cfg, case.bcs)
+
+
+@pytest.mark.parametrize("tol", [1e-1, 1e-2, 1e-3, 1e-4])
+def test_a_converging_gmres_launches_no_more_than_a_capped_one(cb, tol):
+    """A solve that ends at its tolerance after k iterations launches what one
+    capped at k does: no preconditioner application that nothing uses (the
+    residuals of these solves fall evenly enough to see the end coming)."""
+    case = cb.cases.ramp()
+    case.cfg.newton_operator = cb.NEWTON_JACOBIAN_FREE
+    case.cfg.jf_accept = 1.0
+    mesh = cb.HostMesh(case.spec)
+    U0 = cb.cases.perturbed_state(case, mesh.n_cells)
+
+    def step(rel_tol, cap):
+        case.cfg.jf_rel_tol, case.cfg.jf_max_iterations = rel_tol, cap
+        with cb.Solver(mesh, case.cfg, case.bcs) as s:
+            s.set_state(U0)
+            s.evaluate_residual()
+            s.freeze_limiter(True)  # the Jacobian-free operator starts here
+            before = s.launch_count()
+            r = s.newton_step(20.0)
+            assert r.jacobian_free == 1
+            return r.krylov_iterations, s.launch_count() - before
+
+    its, launches = step(tol, 100)
+    assert 1 < its < 100
+    assert step(1e-30, its) == (its, launches)
