@@ -223,7 +223,11 @@ typedef struct cfdg_config {
      * whose conditional while-node repeats the iteration until the device-side
      * state stops it (no host round trip per iteration; profiling switches to
      * the host loop); CFDG_KRYLOV_HOST_LOOP: one launch sequence per
-     * iteration with the host reading the state after each. */
+     * iteration with the host reading the state after each.  With the device
+     * loop a matrix of more than 252 MB (5x5 blocks, or 6x6 in FP32; not where
+     * the solve is reduced, see cfdg_bicgstab) is kept a second time, in the
+     * layout of its sweeps, while eight times its size is free when the copy is
+     * made; the host loop keeps one.  Both give the same bits. */
     int32_t krylov_loop;
     int32_t pre_freeze;       /* CFDG_PREFREEZE_*                             */
     int32_t reserved_;        /* zero                                         */
