@@ -482,8 +482,10 @@ __global__ void k_red_enter(const KrylovScalars* ks, cudaGraphConditionalHandle 
 // where cond(D) is 1e8), coupled stiff terms do.  Limit 8: on matrices whose blocks
 // have 4 to 8, both forms end at the same true residual, 2.6e-16 |b| (the worst
 // 1.25 times the other's); at 16 to 23 the reduced form ends at 1.7 times the
-// full one's, at 90 to 128 at 6 times, at 1e8 at 1e7 times.  Bound by the two
-// reads of n BS^2 values; a lane holds a row of both factors.
+// full one's, at 90 to 128 at 6 times, at 1e8 at 1e7 times.  Bound by L1 wavefronts
+// and shuffles (a lane holds a row of both factors): set-up of 480k rows of 5x5
+// 94 -> 143 us, of 48k 31 -> 33, where an iteration of the solve saves 300 and 30; a
+// thread per block, staged through shared memory, spilled and took 170.
 constexpr double kGrowthLimit = 8.0;
 
 template <int BS>
