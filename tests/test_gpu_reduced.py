@@ -84,7 +84,7 @@ def test_converged_is_the_true_residual(cb, kind, n, bs, order, cond):
 @pytest.mark.parametrize("cond", [1.0, 1e8])
 def test_long_solves(cb, order, cond):
     """More than 32 iterations (the residual is formed from the vector every 32),
-    and the same handle on new values: the verdict is the matrix's."""
+    and the same handle on new values: the form follows the matrix."""
     n, bs = 360, 5
     rp, cl, vals, _ = RS.system("box", n, bs, order)
     rows = np.repeat(np.arange(n), np.diff(rp))
